@@ -14,7 +14,7 @@ LIB_PATH = os.path.join(_HERE, "libhawk_b200.so")
 
 HAWK_F32 = 0
 HAWK_BF16 = 1
-ABI_VERSION = 4
+ABI_VERSION = 5
 
 _P = c_void_p
 # name -> (restype, argtypes); mirrors include/hawk_b200.h one to one
@@ -57,6 +57,11 @@ SIGNATURES = {
     "hawk_gates_bwd": (c_int, [_P] * 8 + [c_size_t, c_int64, c_int, c_int, _P, _P]),
     "hawk_debug_wait_timeout": (c_int, [_P, c_size_t, c_longlong, _P, _P]),
     "hawk_linear_ce_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
+    "hawk_linear_ce_saved_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int, c_int]),
+    "hawk_linear_ce_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
+    "hawk_linear_ce_fwd": (c_int, [_P] * 5 + [c_size_t, _P, c_size_t, c_int64, c_int64, c_int64, c_int, c_int, c_int, _P, _P]),
+    "hawk_linear_ce_bwd": (c_int, [_P, _P, _P, c_size_t, _P, _P, c_int, _P, c_int, _P, c_size_t, c_int64, c_int64, c_int64,
+                                   c_int, c_int, _P, _P]),
     "hawk_linear_ce_fwd_bwd": (c_int, [_P, _P, _P, _P, _P, _P, _P, c_size_t, c_int64, c_int64, c_int64, c_int, _P, _P]),
 }
 

@@ -632,7 +632,7 @@ def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor) -> 
     dact = torch.empty(N, H, dtype=torch.float32, device=act.device)
     ws_bytes = lib.hawk_linear_ce_workspace_bytes(N, H, V)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=act.device)
-    with _on(act, "linear_ce", 9 if weight.dtype == torch.float32 else 7):
+    with _on(act, "linear_ce", 10 if weight.dtype == torch.float32 else 8):
         _lib.check(lib.hawk_linear_ce_fwd_bwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(),
                                               dweight.data_ptr(), dact.data_ptr(), ws.data_ptr(), ws_bytes, N, H, V,
                                               _dt(weight), _status_word(act.device).data_ptr(), _stream(act)),
@@ -646,30 +646,96 @@ def _(weight, act, labels):
             act.new_empty(act.shape, dtype=torch.float32))
 
 
+linear_ce.register_autograd(
+    lambda ctx, g_loss, g_dw, g_da: tuple((g_loss * t).to(dt) for t, dt in zip(ctx.saved_tensors, ctx.dtypes)) + (None,),
+    setup_context=lambda ctx, inputs, output: (ctx.save_for_backward(*output[1:]),
+                                               setattr(ctx, "dtypes", (inputs[0].dtype, inputs[1].dtype)))[0])
+
+
+@torch.library.custom_op("hawk_b200::linear_ce_fwd", mutates_args=())
+def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
+                  want_grad: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(loss [], saved): mean CE(act @ weight^T, labels) and, with want_grad, what linear_ce_bwd needs."""
+    lib = _lib.load()
+    V, H = weight.shape
+    N = act.shape[0]
+    weight, act, labels = weight.contiguous(), act.contiguous(), labels.contiguous()
+    if labels.dtype != torch.int64:
+        labels = labels.long()
+    loss = torch.empty((), dtype=torch.float32, device=act.device)
+    saved = torch.empty(lib.hawk_linear_ce_saved_bytes(N, H, V, _dt(weight), _dt(act)), dtype=torch.uint8, device=act.device)
+    ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
+    casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
+    with _on(act, "linear_ce", 3 + casts + bool(want_grad)):
+        _lib.check(lib.hawk_linear_ce_fwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(),
+                                          saved.data_ptr(), saved.numel(), ws.data_ptr(), ws.numel(), N, H, V, _dt(weight),
+                                          _dt(act), int(want_grad), _status_word(act.device).data_ptr(), _stream(act)),
+                   "hawk_linear_ce_fwd")
+    return loss, saved
+
+
+@linear_ce_fwd.register_fake
+def _(weight, act, labels, want_grad):
+    (V, H), N = weight.shape, act.shape[0]
+    up = lambda n: (n + 255) // 256 * 256
+    n = up(N * ((V + 7) // 8 * 8) * 2)
+    n += up(V * H * 2) if weight.dtype == torch.float32 else 0
+    n += up(N * H * 2) if act.dtype == torch.float32 else 0
+    return act.new_empty((), dtype=torch.float32), act.new_empty(n, dtype=torch.uint8)
+
+
+@torch.library.custom_op("hawk_b200::linear_ce_bwd", mutates_args=())
+def linear_ce_bwd(weight: torch.Tensor, act: torch.Tensor, saved: torch.Tensor, grad_loss: torch.Tensor, want_dw: bool,
+                  want_da: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(d weight, d act) in the operands' dtypes, times grad_loss (empty where not wanted)."""
+    lib = _lib.load()
+    V, H = weight.shape
+    N = act.shape[0]
+    weight, act = weight.contiguous(), act.contiguous()
+    g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
+    dw = torch.empty((V, H) if want_dw else 0, dtype=weight.dtype, device=act.device)
+    da = torch.empty((N, H) if want_da else 0, dtype=act.dtype, device=act.device)
+    ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
+    with _on(act, "linear_ce", 1 + want_dw + want_da):
+        _lib.check(lib.hawk_linear_ce_bwd(weight.data_ptr(), act.data_ptr(), saved.data_ptr(), saved.numel(), g.data_ptr(),
+                                          dw.data_ptr() if want_dw else None, _dt(weight),
+                                          da.data_ptr() if want_da else None, _dt(act), ws.data_ptr(), ws.numel(), N, H, V,
+                                          _dt(weight), _dt(act), _status_word(act.device).data_ptr(), _stream(act)),
+                   "hawk_linear_ce_bwd")
+    return dw, da
+
+
+@linear_ce_bwd.register_fake
+def _(weight, act, saved, grad_loss, want_dw, want_da):
+    return (weight.new_empty(weight.shape if want_dw else 0), act.new_empty(act.shape if want_da else 0))
+
+
 def _ce_setup(ctx, inputs, output):
-    weight, act, _ = inputs
-    _, dweight, dact = output
-    ctx.save_for_backward(dweight, dact)
-    ctx.dtypes = (weight.dtype, act.dtype)
+    weight, act, _, want_grad = inputs
+    assert want_grad, "linear_ce_fwd(want_grad=False) cannot be differentiated"
+    ctx.save_for_backward(weight, act, output[1])
+    ctx.set_materialize_grads(False)
 
 
-def _ce_backward(ctx, g_loss, g_dw, g_da):
-    dweight, dact = ctx.saved_tensors  # computed in the forward, as in the reference (:63,66-73)
-    wd, ad = ctx.dtypes
-    return (g_loss * dweight).to(wd), (g_loss * dact).to(ad), None
+def _ce_backward(ctx, g_loss, g_saved):
+    if g_loss is None:
+        return None, None, None, None
+    want_dw, want_da = ctx.needs_input_grad[:2]
+    dw, da = linear_ce_bwd(*ctx.saved_tensors, g_loss, want_dw, want_da)
+    return dw if want_dw else None, da if want_da else None, None, None
 
 
-linear_ce.register_autograd(_ce_backward, setup_context=_ce_setup)
+linear_ce_fwd.register_autograd(_ce_backward, setup_context=_ce_setup)
 
 
 def fused_cross_entropy(lm_head_weight, act, labels):
     """Mean cross-entropy of `act @ lm_head_weight.T` against `labels`; drop-in for
     hawk/fused_cross_entropy.py:77-79.  weight [V,H], act [N,H] (fp32 or bf16), labels [N] int64.
     The arithmetic is the reference's under bf16 autocast whether or not autocast is on: bf16
-    tensor-core GEMMs with fp32 accumulation, bf16 logits, fp32 softmax."""
-    if act.dtype != lm_head_weight.dtype:
-        act = act.to(lm_head_weight.dtype)
-    return linear_ce(lm_head_weight, act, labels)[0]
+    tensor-core GEMMs with fp32 accumulation, bf16 logits, fp32 softmax.  weight and act may differ in dtype; each
+    gradient has its operand's."""
+    want_grad = torch.is_grad_enabled() and (lm_head_weight.requires_grad or act.requires_grad)
+    return linear_ce_fwd(lm_head_weight, act, labels, want_grad)[0]
 
 
 class CrossEntropyLoopedFused:

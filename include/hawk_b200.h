@@ -28,7 +28,7 @@
 extern "C" {
 #endif
 
-#define HAWK_B200_ABI_VERSION 4
+#define HAWK_B200_ABI_VERSION 5
 
 typedef enum hawk_dtype { HAWK_F32 = 0, HAWK_BF16 = 1 } hawk_dtype;
 
@@ -208,6 +208,21 @@ int hawk_decode_block_step(const void* xy, int64_t xy_row_stride, void* conv_sta
  * it has no ignore_index): a label outside the range makes `loss` non-finite (NaN or inf).
  * ---------------------------------------------------------------------------------------- */
 size_t hawk_linear_ce_workspace_bytes(int64_t N, int64_t H, int64_t V);
+/* The same computation as two calls, as autograd runs it.  hawk_linear_ce_fwd writes the loss and, with want_grad,
+ * leaves dprobs and the bf16 copies of fp32 operands in `saved` (hawk_linear_ce_saved_bytes, 256-byte aligned);
+ * hawk_linear_ce_bwd turns them into dweight [V,H] and dact [N,H] (either may be NULL), in fp32 or bf16, times the
+ * device scalar *grad_loss (NULL: 1).  weight and act are the forward's, in w_dtype / a_dtype (they may differ), and are
+ * read again where they are bf16.  scratch: hawk_linear_ce_scratch_bytes(N, H, V), 256-byte aligned, free after each
+ * call.  An abandoned wait makes the loss, or the first element of each gradient, NaN. */
+size_t hawk_linear_ce_saved_bytes(int64_t N, int64_t H, int64_t V, int w_dtype, int a_dtype);
+size_t hawk_linear_ce_scratch_bytes(int64_t N, int64_t H, int64_t V);
+int hawk_linear_ce_fwd(const void* weight, const void* act, const int64_t* labels, float* loss, void* saved,
+                       size_t saved_bytes, void* scratch, size_t scratch_bytes, int64_t N, int64_t H, int64_t V,
+                       int w_dtype, int a_dtype, int want_grad, int* status, void* stream);
+int hawk_linear_ce_bwd(const void* weight, const void* act, const void* saved, size_t saved_bytes,
+                       const float* grad_loss, void* dweight, int dw_dtype, void* dact, int da_dtype, void* scratch,
+                       size_t scratch_bytes, int64_t N, int64_t H, int64_t V, int w_dtype, int a_dtype, int* status,
+                       void* stream);
 int hawk_linear_ce_fwd_bwd(const void* weight, const void* act, const int64_t* labels, float* loss,
                            float* dweight, float* dact, void* workspace, size_t workspace_bytes,
                            int64_t N, int64_t H, int64_t V, int dtype, int* status, void* stream);
