@@ -18,15 +18,20 @@
 //      behind for it, so no pass over [V,H] or [N,H] fp32 gradients follows the GEMMs.
 //
 // The GEMM is one kernel: C[M,Nc] = A[M,K] . B[Nc,K]^T, bf16 operands, fp32 accumulation.
-// A pair of CTAs (cta_group::2) computes a 256x256 output tile, K in blocks of 64 (128-byte swizzled rows).  What
+// A pair of CTAs (cta_group::2) computes a 256*MH x 256 output tile, K in blocks of 64 (128-byte swizzled rows).  What
 // bounds a CTA working alone on 128x256 is operand delivery from L2: 48 KB per 512 clocks of MMA, 96 B/clk/SM; a
-// pair shares B, 32 KB per CTA in the same time.  Warp-specialised:
-//   warp 0   : TMA producer of its CTA's halves of A and B (cp.async.bulk.tensor, 5-stage ring);
-//   warp 1   : owns TMEM (512 columns = two accumulators); in the leader CTA it issues tcgen05.mma for the pair;
+// pair shares B: 32 KB per CTA in the same time with MH = 1, 24 KB with MH = 2.
+//   MH = 1: two TMEM accumulators, the epilogue overlaps the next tile's MMA: the logits, whose epilogue is long.
+//   MH = 2: the two 256-row halves fill TMEM and share each B tile: the gradient GEMMs when K is long enough for the
+//           epilogue that nothing overlaps (tensor pipe active at N8192 H2048 V8192: 79 % with MH = 1).
+// Warp-specialised:
+//   warp 0   : TMA producer of its CTA's halves of A and B (cp.async.bulk.tensor, ring of 5 or 4 stages);
+//   warp 1   : owns TMEM (512 columns); in the leader CTA it issues tcgen05.mma for the pair;
 //   warps 2-9: epilogue, two warps per TMEM lane quarter (128 columns each), overlapping the next tile's MMA.  The
 //      softmax epilogue is ~10 issue slots and one MUFU operation per logit; with four warps it, not the MMA, set the
-//      pace at H = 512 (N32752 V32000: 1.73 ms for 1.07e12 flop).  bf16 tiles leave through shared memory as TMA box
-//      stores (full 128-byte lines).
+//      pace at H = 512 (N32752 V32000: 1.73 ms for 1.07e12 flop).  Tiles leave through shared memory as TMA box
+//      stores: full 128-byte lines.  (fp32 rows stored 16 bytes per lane ran at 1.5 TB/s: d weight of 777 rows,
+//      V31999 H1024, 92 us.)
 // Persistent over tiles (grid = 2 * min(tiles, SM count / 2)).  Every mbarrier wait is bounded by a clock
 // budget; on expiry the kernel records a status word, drains, frees TMEM and returns.
 #include <algorithm>
@@ -38,11 +43,17 @@ using namespace tc;
 
 constexpr int BM = 256, BN = 256, BK = 64, UMMA_K = 16;  // one tcgen05.mma of the pair covers 256 x 256 x 16
 constexpr int HALF_BYTES = 128 * BK * 2;                 // one CTA's half of an operand tile: 128 M or N indices x 64 K
-constexpr int STAGE_BYTES = 2 * HALF_BYTES;              // A half, then B half
-constexpr int KSTAGES = 5;
 constexpr int EPI_WARPS = 8, EPI_COLS = 128;             // columns of a tile per epilogue warp
-constexpr int BOX_BYTES = 32 * 128;                      // store box: 32 rows x 64 bf16 columns
-constexpr int GEMM_SMEM = KSTAGES * STAGE_BYTES + EPI_WARPS * 2 * BOX_BYTES + 1024;  // + slack for 1024-byte alignment
+constexpr int BOX_BYTES = 32 * 128;                      // store box: 32 rows x 64 bf16 or 32 fp32 columns
+template <int MH>
+struct GemmCfg {
+  static constexpr int STAGES = MH == 1 ? 5 : 4;
+  static constexpr int A_BYTES = MH * HALF_BYTES;               // A halves first, then the B half
+  static constexpr int STAGE_BYTES = A_BYTES + HALF_BYTES;
+  static constexpr int NBOX = MH == 1 ? 2 : 1;                  // store boxes per epilogue warp
+  static constexpr int SMEM = STAGES * STAGE_BYTES + EPI_WARPS * NBOX * BOX_BYTES + 1024;  // + slack for 1024-byte alignment
+  static constexpr int NACC = MH == 1 ? 2 : 1;
+};
 constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
 
 enum { EPI_LOGITS = 0, EPI_OUT = 1 };
@@ -55,10 +66,8 @@ struct EpiParams {
   float* correct;            // [M] logit at the label
   const long long* labels;   // [M]
   // EPI_OUT
-  float* out;                // [M, Nc] fp32, or null when out_bf is the result
-  __nv_bfloat16* out_bf;
+  int out_bf16;              // the store map's type
   const float* scale;        // device scalar multiplied in; null = 1
-  long long split_stride;    // elements between the partial results of consecutive splits
 };
 
 constexpr int MN_BOX = 64 * 128;  // bytes of one [64 columns x 64 rows] box of an MN-major operand
@@ -116,17 +125,43 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t (&v)[32], int cbase
   }
 }
 
+// An epilogue warp's store boxes of 32 rows x 128 bytes (lane = row; 16-byte piece index XOR row mod 8, the store's
+// swizzle), NBOX of them used in turn; every store is one bulk group of lane 0, so that counting groups tells when a box
+// has been read out and may be refilled.
+template <int NBOX>
+__device__ __forceinline__ void box_reuse(int lane) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(NBOX - 1) : "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ void box_put(unsigned char* box, int lane, int piece0, const uint32_t (&p)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    *reinterpret_cast<uint4*>(box + lane * 128 + (((piece0 + q) ^ (lane & 7)) * 16)) =
+        make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+}
+__device__ __forceinline__ void box_store(const CUtensorMap* map, const unsigned char* box, int lane, int col, int row,
+                                          int depth, const EpiParams& ep) {
+  fence_smem_to_tma();
+  __syncwarp();
+  if (lane == 0) {
+    if (col < ep.Nc && row < ep.M) tma_store_3d(map, box, col, row, depth);
+    bulk_commit();  // an empty group where nothing is stored: the group count stays in step
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------------------------
 // A_MN / B_MN: the operand is read as an MN-major tile, i.e. straight from a row-major [K, M] (or [K, Nc])
 // tensor whose rows are the contraction index; its tensor map then has boxes of [64 columns x 64 rows],
 // one box per 64 M/N indices, 8192 bytes apart in the stage.
-template <int MODE, bool A_MN, bool B_MN>
+template <int MODE, int MH, bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_c, int K, int m_tiles, int n_tiles, int splits, EpiParams ep,
                  int* status) {
+  using Cfg = GemmCfg<MH>;
+  constexpr int KSTAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES, A_BYTES = Cfg::A_BYTES, NACC = Cfg::NACC;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full_bar[KSTAGES], empty_bar[KSTAGES], tfull_bar[2], tempty_bar[2];
@@ -168,7 +203,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         int mt, nt;
         tile_coords(tile % tiles, m_tiles, n_tiles, mt, nt);
         const int kb0 = (tile / tiles) * ep.k_per_split, kb1 = min(kblocks, kb0 + ep.k_per_split);
-        const int m0 = mt * BM + (int)rank * 128, n0 = nt * BN + (int)rank * 128;
+        const int m0 = mt * BM * MH + (int)rank * 128, n0 = nt * BN + (int)rank * 128;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % KSTAGES;
           const uint32_t ph = (it / KSTAGES) & 1;
@@ -176,17 +211,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
           const uint32_t bar = map_to_rank(&full_bar[s], 0);
           unsigned char* st = smem + s * STAGE_BYTES;
-          if (A_MN) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) tma_load_2d_pair(st + q * MN_BOX, &map_a, bar, m0 + q * 64, kb * BK);
-          } else {
-            tma_load_2d_pair(st, &map_a, bar, kb * BK, m0);
+          for (int hh = 0; hh < MH; ++hh) {
+            if (A_MN) {
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+                tma_load_2d_pair(st + hh * HALF_BYTES + q * MN_BOX, &map_a, bar, m0 + hh * BM + q * 64, kb * BK);
+            } else {
+              tma_load_2d_pair(st + hh * HALF_BYTES, &map_a, bar, kb * BK, m0 + hh * BM);
+            }
           }
           if (B_MN) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) tma_load_2d_pair(st + HALF_BYTES + q * MN_BOX, &map_b, bar, n0 + q * 64, kb * BK);
+            for (int q = 0; q < 2; ++q) tma_load_2d_pair(st + A_BYTES + q * MN_BOX, &map_b, bar, n0 + q * 64, kb * BK);
           } else {
-            tma_load_2d_pair(st + HALF_BYTES, &map_b, bar, kb * BK, n0);
+            tma_load_2d_pair(st + A_BYTES, &map_b, bar, kb * BK, n0);
           }
         }
       }
@@ -202,8 +241,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (lane == 0 && rank == 0) {
       uint32_t it = 0, tcount = 0;
       for (int tile = first_tile; tile < num_tiles && !*abortp; tile += tile_stride, ++tcount) {
-        const int acc = tcount & 1;
-        if (!mbar_wait(&tempty_bar[acc], ((tcount >> 1) & 1) ^ 1, abortp)) break;
+        const int acc = NACC == 2 ? (tcount & 1) : 0;
+        const uint32_t aph = NACC == 2 ? ((tcount >> 1) & 1) : (tcount & 1);
+        if (!mbar_wait(&tempty_bar[acc], aph ^ 1, abortp)) break;
         fence_after();
         const int kb0 = (tile / tiles) * ep.k_per_split, kb1 = min(kblocks, kb0 + ep.k_per_split);
         const uint32_t d_tmem = tmem_base + acc * BN;
@@ -214,13 +254,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (!mbar_wait(&full_bar[s], ph, abortp)) { ok = false; break; }
           fence_after();
           const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + HALF_BYTES;
+          const uint32_t b_addr = a_addr + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // K-major: 16 K-elements further along the 128-byte rows; MN-major: 16 K-rows (2048 bytes) further down
-            const uint64_t ad = A_MN ? umma_desc_sw128(a_addr + k * UMMA_K * 128, MN_BOX) : umma_desc_sw128(a_addr + k * UMMA_K * 2);
             const uint64_t bd = B_MN ? umma_desc_sw128(b_addr + k * UMMA_K * 128, MN_BOX) : umma_desc_sw128(b_addr + k * UMMA_K * 2);
-            umma_bf16_pair(d_tmem, ad, bd, kIdescMaj, (kb > kb0 || k > 0) ? 1u : 0u);
+#pragma unroll
+            for (int hh = 0; hh < MH; ++hh) {
+              const uint32_t ah = a_addr + hh * HALF_BYTES;
+              const uint64_t ad = A_MN ? umma_desc_sw128(ah + k * UMMA_K * 128, MN_BOX) : umma_desc_sw128(ah + k * UMMA_K * 2);
+              umma_bf16_pair(d_tmem + hh * BN, ad, bd, kIdescMaj, (kb > kb0 || k > 0) ? 1u : 0u);
+            }
           }
           umma_commit_pair(&empty_bar[s]);  // frees the stage in both CTAs once these MMAs have read it
         }
@@ -232,20 +276,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // ---------------- epilogue (warps 2..9) ----------------
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 are the ones this warp may read
     const int half = (warp - 2) >> 2;
-    unsigned char* boxes = smem + KSTAGES * STAGE_BYTES + (warp - 2) * 2 * BOX_BYTES;
+    unsigned char* boxes = smem + KSTAGES * STAGE_BYTES + (warp - 2) * Cfg::NBOX * BOX_BYTES;
     const float scale = (MODE == EPI_OUT && ep.scale) ? *ep.scale : 1.f;
     uint32_t tcount = 0;
     for (int tile = first_tile; tile < num_tiles; tile += tile_stride, ++tcount) {
       if (*abortp) break;
       int mt, nt;
       tile_coords(tile % tiles, m_tiles, n_tiles, mt, nt);
-      const int acc = tcount & 1;
-      if (!mbar_wait_warp(&tfull_bar[acc], (tcount >> 1) & 1, abortp)) break;  // lane 0 waits: the warp cannot diverge
+      const int acc = NACC == 2 ? (tcount & 1) : 0;
+      if (!mbar_wait_warp(&tfull_bar[acc], NACC == 2 ? ((tcount >> 1) & 1) : (tcount & 1), abortp)) break;  // lane 0 waits: the warp cannot diverge
       fence_after();
       const int col0 = nt * BN + half * EPI_COLS;
-      const int row0 = mt * BM + (int)rank * 128 + quarter * 32, row = row0 + lane;
+#pragma unroll 1
+      for (int hh = 0; hh < MH; ++hh) {
+      const int row0 = (mt * MH + hh) * BM + (int)rank * 128 + quarter * 32, row = row0 + lane;
       const bool row_ok = row < ep.M;
-      const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * EPI_COLS);
+      const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((acc + hh) * BN + half * EPI_COLS);
       uint32_t v[2][32];
       tmem_ld32_async(taddr0, v[0]);
 
@@ -268,65 +314,54 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           }
           // box c/2 of the warp: 32 rows x 64 columns, 16-byte piece index XOR row mod 8 (the store's swizzle)
           unsigned char* box = boxes + (c >> 1) * BOX_BYTES;
-          if ((c & 1) == 0) {  // the box is about to be refilled: its previous store must have read it
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            __syncwarp();
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int piece = ((c & 1) * 4 + q) ^ (lane & 7);
-            *reinterpret_cast<uint4*>(box + lane * 128 + piece * 16) =
-                make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-          }
-          if (c & 1) {
-            fence_smem_to_tma();
-            __syncwarp();
-            if (lane == 0) {
-              const int bc = col0 + (c >> 1) * 64;
-              if (bc < ep.Nc && row0 < ep.M) tma_store_2d(&map_c, box, bc, row0);
-              bulk_commit();  // an empty group where nothing is stored: the group count stays in step
-            }
-          }
+          if ((c & 1) == 0) box_reuse<2>(lane);
+          box_put(box, lane, (c & 1) * 4, packed);
+          if (c & 1) box_store(&map_c, box, lane, col0 + (c >> 1) * 64, row0, 0, ep);
         }
         if (row_ok && col0 < ep.Nc) ep.stats[(long long)(col0 / EPI_COLS) * ep.M + row] = make_float2(run_m, run_s);
       } else {
-        const long long o = (long long)(tile / tiles) * ep.split_stride + (long long)(row_ok ? row : 0) * ep.Nc + col0;
-#pragma unroll
-        for (int c = 0; c < EPI_COLS / 32; ++c) {
+        const int split = tile / tiles;
+        auto chunk = [&](int c) -> const uint32_t(&)[32] {  // waits for chunk c, requests the next one
           tmem_ld_wait();
           if (c + 1 < EPI_COLS / 32) tmem_ld32_async(taddr0 + (c + 1) * 32, v[(c + 1) & 1]);
-          const int cbase = col0 + c * 32;
-          if (row_ok && cbase < ep.Nc) {
-            const uint32_t(&w)[32] = v[c & 1];
-            if (ep.out_bf != nullptr) {
-              __nv_bfloat16* orow = ep.out_bf + o + c * 32;
+          return v[c & 1];
+        };
+        if (ep.out_bf16) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q)  // Nc is a multiple of 8: whole 16-byte pieces
-                if (cbase + q * 8 < ep.Nc) {
-                  uint4 p;
-                  p.x = pack_bf16x2(__uint_as_float(w[8 * q]) * scale, __uint_as_float(w[8 * q + 1]) * scale);
-                  p.y = pack_bf16x2(__uint_as_float(w[8 * q + 2]) * scale, __uint_as_float(w[8 * q + 3]) * scale);
-                  p.z = pack_bf16x2(__uint_as_float(w[8 * q + 4]) * scale, __uint_as_float(w[8 * q + 5]) * scale);
-                  p.w = pack_bf16x2(__uint_as_float(w[8 * q + 6]) * scale, __uint_as_float(w[8 * q + 7]) * scale);
-                  *reinterpret_cast<uint4*>(orow + q * 8) = p;
-                }
-            } else {
-              float* orow = ep.out + o + c * 32;
+          for (int c = 0; c < EPI_COLS / 32; ++c) {
+            const uint32_t(&w)[32] = chunk(c);
+            uint32_t packed[16];
 #pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (cbase + q * 4 < ep.Nc)
-                  *reinterpret_cast<float4*>(orow + q * 4) =
-                      make_float4(__uint_as_float(w[4 * q]) * scale, __uint_as_float(w[4 * q + 1]) * scale,
-                                  __uint_as_float(w[4 * q + 2]) * scale, __uint_as_float(w[4 * q + 3]) * scale);
+            for (int j = 0; j < 16; ++j)
+              packed[j] = pack_bf16x2(__uint_as_float(w[2 * j]) * scale, __uint_as_float(w[2 * j + 1]) * scale);
+            unsigned char* box = boxes + ((c >> 1) % Cfg::NBOX) * BOX_BYTES;
+            if ((c & 1) == 0) box_reuse<Cfg::NBOX>(lane);
+            box_put(box, lane, (c & 1) * 4, packed);
+            if (c & 1) box_store(&map_c, box, lane, col0 + (c >> 1) * 64, row0, split, ep);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < EPI_COLS / 32; ++c) {
+            const uint32_t(&w)[32] = chunk(c);
+            unsigned char* box = boxes + (c % Cfg::NBOX) * BOX_BYTES;
+            box_reuse<Cfg::NBOX>(lane);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              uint32_t scaled[16];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) scaled[j] = __float_as_uint(__uint_as_float(w[16 * q + j]) * scale);
+              box_put(box, lane, q * 4, scaled);
             }
+            box_store(&map_c, box, lane, col0 + c * 32, row0, split, ep);
           }
         }
       }
+      }  // halves
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_rank(&tempty_bar[acc], 0));
     }
-    if (MODE == EPI_LOGITS && lane == 0) bulk_wait_all();
+    if (lane == 0) bulk_wait_all();
   }
 
   // ---------------- teardown ----------------
@@ -460,22 +495,22 @@ ce_dprobs_kernel(__nv_bfloat16* __restrict__ logits, long long ldl, const float*
 // ---------------------------------------------------------------------------------------------
 // C[M, Nc] = A . B^T with bf16 operands.  A K-major operand is a row-major [M, K] (or [Nc, K]) tensor; an
 // MN-major operand (A_MN / B_MN) is a row-major [K, M] (or [K, Nc]) tensor.  lda / ldb: row pitches.
-template <int MODE, bool A_MN, bool B_MN>
-static int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb, __nv_bfloat16* C,
+template <int MODE, int MH, bool A_MN, bool B_MN>
+static int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb, void* C, bool c_f32,
                        long long ldc, int M, int Nc, int K, int splits, EpiParams ep, int* status, cudaStream_t st) {
   CUtensorMap ma, mb, mc;
   const bool oka = A_MN ? make_map_bf16(&ma, A, K, M, lda, 64) : make_map_bf16(&ma, A, M, K, lda, 128);
   const bool okb = B_MN ? make_map_bf16(&mb, B, K, Nc, ldb, 64) : make_map_bf16(&mb, B, Nc, K, ldb, 128);
   if (!oka || !okb) return HAWK_ERR_DEVICE;
-  mc = ma;  // not used by EPI_OUT
-  if (MODE == EPI_LOGITS && !make_map_bf16(&mc, C, M, Nc, ldc, 32)) return HAWK_ERR_DEVICE;
-  auto kern = gemm_bf16_kernel<MODE, A_MN, B_MN>;
+  if (!make_map_store(&mc, C, c_f32, Nc, M, splits, ldc, (long long)M * ldc)) return HAWK_ERR_DEVICE;
+  auto kern = gemm_bf16_kernel<MODE, MH, A_MN, B_MN>;
+  constexpr int GEMM_SMEM = GemmCfg<MH>::SMEM;
   // per call: the attribute belongs to the current device's copy of the kernel
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess) {
     (void)cudaGetLastError();
     return HAWK_ERR_LAUNCH;
   }
-  const int m_tiles = (M + BM - 1) / BM, n_tiles = (Nc + BN - 1) / BN, kblocks = (K + BK - 1) / BK;
+  const int m_tiles = (M + BM * MH - 1) / (BM * MH), n_tiles = (Nc + BN - 1) / BN, kblocks = (K + BK - 1) / BK;
   ep.M = M;
   ep.Nc = Nc;
   ep.k_per_split = (kblocks + splits - 1) / splits;
@@ -485,23 +520,29 @@ static int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   return launch_status();
 }
 
-// K splits of a gradient GEMM.  With few output tiles most CTA pairs would idle (d act of 1548 rows at H = 512: 14
-// tiles on 74 pairs, 310 us); cost in K-block times (0.27 us each): waves x (K blocks per split + 12 for the tile's
-// fill and epilogue) + the pass that sums the partials.  No split is left without K blocks.
-static int choose_splits(long long M, long long Nc, long long K) {
-  const long long tiles = ((M + BM - 1) / BM) * ((Nc + BN - 1) / BN), kb = (K + BK - 1) / BK;
-  const long long pairs = std::max(1, sm_count() / 2);
-  int best = 1;
-  double best_cost = 0;
-  for (int s = 1; s <= 32 && s <= kb; ++s) {
-    const long long per = (kb + s - 1) / s;
-    if ((s - 1) * per >= kb) continue;
-    const double waves = (double)((tiles * s + pairs - 1) / pairs);
-    const double sum_us = s > 1 ? 4.0 + 4.0 * (double)M * Nc * (s + 1) / 5.0e6 : 0.0;
-    const double cost = waves * (double)(per + 12) + sum_us / 0.27;
-    if (s == 1 || cost < best_cost) {
-      best = s;
-      best_cost = cost;
+// Tile height (MH) and K splits of a gradient GEMM.  With few output tiles most CTA pairs would idle (d act of 1548
+// rows at H = 512: 14 tiles of 256 rows on 74 pairs, 310 us unsplit), so K is split; a K block costs 0.37 us with
+// MH = 1 and 0.58 us with MH = 2 (two halves), a tile about 5 and 9 us of fill and epilogue, and splits a pass that
+// sums the partials.  No split is left without K blocks.
+struct GradPlan {
+  int mh, splits;
+};
+static GradPlan plan_grad(long long M, long long Nc, long long K) {
+  const long long kb = (K + BK - 1) / BK, pairs = std::max(1, sm_count() / 2);
+  GradPlan best{1, 1};
+  double best_us = 0;
+  for (int mh = 1; mh <= 2; ++mh) {
+    const long long tiles = ((M + BM * mh - 1) / (BM * mh)) * ((Nc + BN - 1) / BN);
+    for (int s = 1; s <= 32 && s <= kb; ++s) {
+      const long long per = (kb + s - 1) / s;
+      if ((s - 1) * per >= kb) continue;
+      const double waves = (double)((tiles * s + pairs - 1) / pairs);
+      const double sum_us = s > 1 ? 4.0 + 4.0 * (double)M * Nc * (s + 1) / 5.0e6 : 0.0;
+      const double us = waves * (mh == 1 ? per * 0.37 + 5.0 : per * 0.58 + 9.0) + sum_us;
+      if (best_us == 0 || us < best_us) {
+        best = GradPlan{mh, s};
+        best_us = us;
+      }
     }
   }
   return best;
@@ -542,7 +583,7 @@ static CeScratch ce_fwd_scratch(long long N, long long V) {
   return L;
 }
 static size_t ce_bwd_scratch(long long N, long long H, long long V) {  // the two GEMMs run one after the other
-  const int sa = choose_splits(N, H, V), sw = choose_splits(V, H, N);
+  const int sa = plan_grad(N, H, V).splits, sw = plan_grad(V, H, N).splits;
   return std::max(sa > 1 ? up256((size_t)sa * N * H * 4) : 0, sw > 1 ? up256((size_t)sw * V * H * 4) : 0);
 }
 
@@ -557,17 +598,15 @@ static int check_ce(int64_t N, int64_t H, int64_t V, int w_dtype, int a_dtype) {
 template <bool A_MN, bool B_MN>
 static int grad_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb, void* out, int out_dtype,
                      const float* scale, int M, int Nc, int K, float* scratch, int* status, cudaStream_t st) {
-  const int splits = choose_splits(M, Nc, K);
+  const GradPlan plan = plan_grad(M, Nc, K);
+  const int splits = plan.splits;
   EpiParams ep{};
-  if (splits > 1) {
-    ep.out = scratch;
-    ep.split_stride = (long long)M * Nc;
-  } else {
-    if (out_dtype == HAWK_BF16) ep.out_bf = static_cast<__nv_bfloat16*>(out);
-    else ep.out = static_cast<float*>(out);
-    ep.scale = scale;
-  }
-  int rc = launch_gemm<EPI_OUT, A_MN, B_MN>(A, lda, B, ldb, nullptr, 0, M, Nc, K, splits, ep, status, st);
+  void* C = splits > 1 ? scratch : out;
+  ep.out_bf16 = splits == 1 && out_dtype == HAWK_BF16;
+  ep.scale = splits > 1 ? nullptr : scale;
+  int rc = plan.mh == 2
+               ? launch_gemm<EPI_OUT, 2, A_MN, B_MN>(A, lda, B, ldb, C, !ep.out_bf16, Nc, M, Nc, K, splits, ep, status, st)
+               : launch_gemm<EPI_OUT, 1, A_MN, B_MN>(A, lda, B, ldb, C, !ep.out_bf16, Nc, M, Nc, K, splits, ep, status, st);
   if (rc != HAWK_OK || splits == 1) return rc;
   const long long n = (long long)M * Nc;
   const unsigned blocks = (unsigned)((n / 4 + 255) / 256);
@@ -642,7 +681,7 @@ extern "C" int hawk_linear_ce_fwd(const void* weight, const void* act, const int
   ep.stats = stats;
   ep.correct = correct;
   ep.labels = reinterpret_cast<const long long*>(labels);
-  rc = launch_gemm<EPI_LOGITS, false, false>(ab, H, wb, H, logits, S.ldV, (int)N, (int)V, (int)H, 1, ep, status, st);
+  rc = launch_gemm<EPI_LOGITS, 1, false, false>(ab, H, wb, H, logits, false, S.ldV, (int)N, (int)V, (int)H, 1, ep, status, st);
   if (rc != HAWK_OK) return rc;
   // 3. log-sum-exp per row and the mean loss
   ce_row_reduce_kernel<<<L.n_blocks, 256, 0, st>>>(stats, correct, lse, partial, (int)N, L.groups);
