@@ -249,11 +249,20 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// Encoding needs a current context.  A thread that has made no runtime call that creates one (autograd's backward thread,
+// when its allocations come from the caching allocator's pool) has none, although its current device is set.
+inline void bind_context() {
+  static thread_local int bound = -1;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev != bound && cudaSetDevice(dev) == cudaSuccess) bound = dev;
+}
+
 // 2-D bf16 tensor [rows, cols] with row pitch ld (elements); box = [box_rows, 64 cols], 128-byte swizzle,
 // out-of-range elements read as zero.  Base 16-byte aligned, ld a multiple of 8.
 inline bool make_map_bf16(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
+  bind_context();
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
   cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
@@ -269,6 +278,7 @@ inline bool make_map_store(CUtensorMap* map, const void* base, bool f32, long lo
                            long long ld, long long depth_stride) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
+  bind_context();
   const cuuint64_t es = f32 ? 4 : 2;
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)depth};
   cuuint64_t strides[2] = {(cuuint64_t)ld * es, (cuuint64_t)depth_stride * es};

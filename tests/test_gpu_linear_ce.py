@@ -121,3 +121,28 @@ def test_label_outside_the_vocabulary_is_visible_in_the_loss():
     labels[17] = 300
     assert not bool(torch.isfinite(ops.fused_cross_entropy(w, act, labels)))
     ops.check_device_status()
+
+
+def test_backward_as_a_threads_first_cuda_call():
+    """The backward runs on autograd's thread, where it can be the first call that needs a context (its buffers come from the
+    allocator's pool): the tensor maps must not fail to encode there."""
+    import threading
+
+    import hawk_b200.ops as ops
+    torch.manual_seed(0)
+    w, act = torch.randn(1000, 64, device="cuda"), torch.randn(300, 64, device="cuda")
+    labels = torch.randint(0, 1000, (300,), device="cuda")
+    _, saved = ops.linear_ce_fwd(w, act, labels, True)
+    one = torch.ones((), device="cuda")
+    want = ops.linear_ce_bwd(w, act, saved, one, True, True)
+    got = []
+    stream = torch.cuda.current_stream()
+    torch.cuda.synchronize()
+
+    def run():
+        with torch.cuda.stream(stream):
+            got.extend(ops.linear_ce_bwd(w, act, saved, one, True, True))
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    assert len(got) == 2 and all(torch.equal(a, b) for a, b in zip(got, want))
