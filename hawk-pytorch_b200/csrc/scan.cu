@@ -857,21 +857,32 @@ static int launch_bwd(const void* x, const void* gx, const void* ga, const float
   return launch_status();
 }
 
-// Launch shape.  A CTA scans all of T for its channel group, so the grid is B * D / CW CTAs of equal
-// cost.  Measured on B200 (bf16), alone and inside a training step (where the SM clock sits near
-// 1.55 GHz under the board's power limit and the kernels turn compute bound): the forward is best
-// with narrow groups (CW = 16: 128-thread CTAs, ~7 per SM, even load on every SM; 256-thread CTAs when
-// there are few groups, e.g. one long sequence: B1 T65536 D4096 4.16 against 4.03 TB/s), the backward
-// with CW = 64 and 8 rows per slot when there are at least ~200 (batch x 64-channel group) pairs, else
-// with CW = 32 to double the CTA count.  (512-thread CTAs measured slower in both directions; backward
-// shapes with 4 rows per slot at 3 CTAs per SM, 78 registers, measured 264-266 us inside the step against
-// 254 us for the 8-row shape at 2 CTAs per SM.)  With few groups the backward runs CW = 32 with 8 rows per
-// slot (B1 T65536 D4096: 0.960 against 1.038 ms for 4 rows and 4 stages).  The fused-epilogue kernels carry
-// more arithmetic per byte and come out best with CW = 32 in both directions where CW = 16 wins for the
-// plain forward: inside the training step 186 against 224 us forward (CW = 32 x 8 rows, 105 registers,
-// 4 CTAs per SM, against CW = 16 at 6 CTAs per SM), 0.750 against 0.914 ms at B1 T65536 D4096; eight other
-// forward shapes and eight backward shapes measured slower inside the step.
+// Launch shape.  A CTA scans all of T for its channel group, so the grid is B * D / CW CTAs of equal cost and what matters is
+// how evenly they fill the 148 SMs and how many rows are in flight on each.  Measured on B200, bf16, L2 flushed, us (R rows
+// per slot x warps x CW):
+//   plain forward                        8x4x32   8x8x32   16x4x16   (before: 8x4x16 / 8x8x16)
+//     B16 T4096 D2048  (1024 groups of 32)  187      195       232      236
+//     B8  T4096 D2048   (512)               109      116       128      126
+//     B16 T2048 D512    (256)                45       38        48       53
+//     B5  T3001 D1536   (240)                59       50        58       62
+//     B1  T65536 D4096  (128)               793      568       507      523
+//     B2  T16384 D2048  (128)               207      151       139      144
+//     B1  T16384 D1024 and other few groups: as 16x4x16, or the time split below
+//   so: 4 warps of CW = 32 where 400 or more CTAs come of it (four fit an SM), 8 warps of CW = 32 where they still reach
+//   every SM, else CW = 16 with 16 rows per slot.
+//   plain backward                       8x8x64   8x8x32   8x16x32
+//     B8  T4096 D2048                       204      216       239
+//     B5  T3001 D1536                        89       89        99
+//     B1  T65536 D4096                     1629      968       884   (fused epilogue: 1250 -> 1164)
+//     B2  T16384 D2048                      417      253       233   (fused epilogue:  323 ->  302)
+//     B4  T2000 D768     (96)                63       44        42   (fused epilogue:   52 ->   54)
+//   so: CW = 64 with 8 warps from 200 of its groups on, CW = 32 below; one CTA of 16 warps instead of one of 8 where there is
+//   at most one per SM and the sequence is long enough for the larger super-steps.
+// The fused-epilogue kernels carry more arithmetic per byte: CW = 32 in the forward throughout (inside the training step
+// 186 against 224 us for CW = 16, at B8 T4096 D2048), otherwise the same lines.
 static bool many_groups(int B, int D) { return (int64_t)B * (D / 64) >= 200; }
+static int64_t groups32(int B, int D) { return (int64_t)B * (D / 32); }
+constexpr int kSms = 148;
 
 static int check_scan_common(int B, int T, int D, int dtype) {
   HAWK_REQUIRE(valid_dtype(dtype), HAWK_ERR_DTYPE);
@@ -910,8 +921,9 @@ static int scan_fwd_dispatch(const void* x, const void* gx, const void* ga, cons
       if (many) HAWK_FWD(bf, 8, 4, 16, 2, 4, true, true);
       HAWK_FWD(bf, 8, 8, 16, 2, 2, true, true);
     }
-    if (many) HAWK_FWD(bf, 8, 4, 8, 2, 7, true, false);
-    HAWK_FWD(bf, 8, 8, 8, 4, 2, true, false);
+    if (many) HAWK_FWD(bf, 8, 4, 16, 2, 4, true, false);
+    if (groups32(B, D) > kSms) HAWK_FWD(bf, 8, 8, 16, 2, 2, true, false);
+    HAWK_FWD(bf, 16, 4, 8, 2, 4, true, false);
   }
   if (ge) HAWK_FWD(float, 4, 4, 8, 4, 3, false, true);
   HAWK_FWD(float, 4, 4, 8, 4, 4, false, false);
@@ -943,13 +955,15 @@ static int scan_bwd_dispatch(const void* x, const void* gx, const void* ga, cons
   return launch_bwd<TT, R, W, LPR, S, MINB, FAST, GELU>(x, gx, ga, lam, h0, gate_bias, h, go, dx, dgx, dga, dlam, dh0, \
                                                         dgate_bias, partial, B, T, D, ge ? *ge : none, st,            \
                                                         split ? *split : whole)
-  const bool many = many_groups(B, D);
+  const bool many = many_groups(B, D), one_per_sm = groups32(B, D) > kSms / 2 && groups32(B, D) <= kSms;
   if (dtype == HAWK_BF16) {
     if (ge) {
       if (many) HAWK_BWD(bf, 8, 8, 32, 2, 2, true, true);
+      if (one_per_sm && T >= 4096) HAWK_BWD(bf, 8, 16, 16, 2, 1, true, true);
       HAWK_BWD(bf, 8, 8, 16, 2, 2, true, true);
     }
     if (many) HAWK_BWD(bf, 8, 8, 32, 2, 2, true, false);
+    if (one_per_sm && T >= 4096) HAWK_BWD(bf, 8, 16, 16, 2, 1, true, false);
     HAWK_BWD(bf, 8, 8, 16, 2, 2, true, false);
   }
   if (ge) {

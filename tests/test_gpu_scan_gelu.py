@@ -118,3 +118,13 @@ def test_fused_scan_gelu_metric_shape_properties():
                               lam[ch].cpu(), compute=torch.float64)
     want = F.gelu(xy[..., D:][..., ch].double().cpu()) * hw
     assert rel_l2(out[..., ch].float().cpu(), want) <= 2e-2
+
+
+def test_long_sequence_of_few_groups():
+    """The 16-warp backward (80 groups of 32 channels, over 4096 rows), with a ragged last super-step."""
+    args = _inputs(1, 4099, 2560, 5, torch.bfloat16)
+    got = _run(*args, torch.bfloat16, True)
+    x, gx, ga, dout, xy, gb, lam = args
+    want = _oracle(x, gx, ga, dout, xy[..., 2560:], gb, lam, got["h"])
+    for k, v in want.items():
+        assert rel_l2(got[k], v) <= 2e-2 and max_rel(got[k], v) <= 2e-2, k
