@@ -24,6 +24,50 @@ inline bool valid_dtype(int d) { return d == HAWK_F32 || d == HAWK_BF16; }
 inline size_t dtype_size(int d) { return d == HAWK_BF16 ? 2 : 4; }
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? HAWK_OK : HAWK_ERR_LAUNCH; }
 
+// ---- programmatic dependent launch --------------------------------------------------------
+// A kernel launched with `pdl` may start while the kernel before it on the stream is still running.  Until its
+// pdl_wait() returns it may read only what that kernel does not write, and it may write nothing; pdl_wait() returns when
+// every earlier kernel has completed and its writes are visible.  pdl_trigger() lets the NEXT such kernel start; it always
+// comes after pdl_wait(), so that a kernel that starts early knows everything before its predecessor to be complete.
+// Both do nothing in a kernel launched in the ordinary way.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Loads of what the preceding kernel wrote: volatile, so that none is moved above pdl_wait() (a load through a
+// const __restrict__ pointer counts as invariant and may be)
+__device__ __forceinline__ uint4 ld_dep16(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
+
+template <typename... KArgs, typename... Args>
+inline int launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
+                         unsigned cluster, Args... args) {
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  if (pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return HAWK_ERR_LAUNCH;
+  }
+  return launch_status();
+}
+
 // ---- two adjacent channels ----------------------------------------------------------------
 // bf16 -> fp32 is a 16-bit shift, so a packed pair unpacks with one shift and one mask.
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {

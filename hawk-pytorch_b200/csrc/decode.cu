@@ -6,7 +6,7 @@
 // block-diagonal gate GEMMs.  Both are one read and one write of [B,D]-sized state: HBM/launch bound.
 #include <type_traits>
 
-#include "common.cuh"
+#include "decode.cuh"
 
 namespace hawk {
 
@@ -100,6 +100,29 @@ decode_block_step_kernel(const T* __restrict__ xy, int64_t ld_xy, TS* __restrict
   TW* ws = reinterpret_cast<TW*>(g + (size_t)2 * kDecTB * bw);  // [2][bw][bw] the block's two weight matrices
   const int blk = blockIdx.x, b0 = blockIdx.y * kDecTB, ch0 = blk * bw;
 
+  // both weight matrices of the block to shared memory, in flight while the other inputs are (and, in a chain of launches,
+  // while the kernel before this one finishes)
+  {
+    const int nel = bw * bw;
+    const TW* src0 = wx + (int64_t)blk * nel;
+    const TW* src1 = wa + (int64_t)blk * nel;
+    const int n16 = nel * (int)sizeof(TW) / 16;
+    if ((nel * (int)sizeof(TW)) % 16 == 0 && (reinterpret_cast<uintptr_t>(src0) % 16) == 0 &&
+        (reinterpret_cast<uintptr_t>(src1) % 16) == 0) {
+      for (int i = threadIdx.x; i < n16; i += blockDim.x) {
+        copy_async16(reinterpret_cast<uint4*>(ws) + i, reinterpret_cast<const uint4*>(src0) + i);
+        copy_async16(reinterpret_cast<uint4*>(ws + nel) + i, reinterpret_cast<const uint4*>(src1) + i);
+      }
+    } else {
+      for (int i = threadIdx.x; i < nel; i += blockDim.x) {
+        ws[i] = src0[i];
+        ws[nel + i] = src1[i];
+      }
+    }
+  }
+  pdl_wait();
+  pdl_trigger();
+
   // Every global input of the launch is requested before anything waits: a thread owns up to kDecIT
   // (batch row, channel) elements (TB * bw <= 256 * kDecIT since bw <= 128) and loads their conv window,
   // new input, y, state and per-channel constants into registers in one unrolled pass, so the kernel pays
@@ -119,46 +142,20 @@ decode_block_step_kernel(const T* __restrict__ xy, int64_t ld_xy, TS* __restrict
     win[it][0] = win[it][1] = win[it][2] = 0.f;
     if (ok[it]) {
       const T* xr = xy + (int64_t)bg * ld_xy;
-      xn[it] = to_float(xr[ch]);
-      yv[it] = to_float(xr[R + ch]);
-      sv[it] = to_float(state[(int64_t)bg * R + ch]);
+      xn[it] = load_dep(xr + ch);
+      yv[it] = load_dep(xr + R + ch);
+      sv[it] = load_dep(state + (int64_t)bg * R + ch);
       lv[it] = lam[ch];
       const TS* sp = conv_state + ((int64_t)bg * (W - 1)) * R + ch;
       float acc = fmaf(cw[(int64_t)(W - 1) * R + ch], xn[it], cb[ch]);
 #pragma unroll
       for (int j = 0; j < 3; ++j) {  // state row j is x[t-(W-1)+j], paired with w[j]
         if (j < W - 1) {
-          win[it][j] = to_float(sp[(int64_t)j * R]);
+          win[it][j] = load_dep(sp + (int64_t)j * R);
           acc = fmaf(cw[(int64_t)j * R + ch], win[it][j], acc);
         }
       }
       cacc[it] = acc;
-    }
-  }
-
-  // stage both weight matrices of the block in shared memory (16-byte copies, all in flight at once)
-  {
-    const int nel = bw * bw;
-    const TW* src0 = wx + (int64_t)blk * nel;
-    const TW* src1 = wa + (int64_t)blk * nel;
-    const bool vec = (nel * (int)sizeof(TW)) % 16 == 0 && (reinterpret_cast<uintptr_t>(src0) % 16) == 0 &&
-                     (reinterpret_cast<uintptr_t>(src1) % 16) == 0;
-    if (vec) {
-      const int n16 = nel * (int)sizeof(TW) / 16;
-      const uint4* s0 = reinterpret_cast<const uint4*>(src0);
-      const uint4* s1 = reinterpret_cast<const uint4*>(src1);
-      uint4* d0 = reinterpret_cast<uint4*>(ws);
-      uint4* d1 = reinterpret_cast<uint4*>(ws + nel);
-#pragma unroll 4
-      for (int i = threadIdx.x; i < n16; i += blockDim.x) {
-        d0[i] = __ldg(s0 + i);
-        d1[i] = __ldg(s1 + i);
-      }
-    } else {
-      for (int i = threadIdx.x; i < nel; i += blockDim.x) {
-        ws[i] = src0[i];
-        ws[nel + i] = src1[i];
-      }
     }
   }
 
@@ -175,33 +172,43 @@ decode_block_step_kernel(const T* __restrict__ xy, int64_t ld_xy, TS* __restrict
       if (W > 1) sp[(int64_t)(W - 2) * R] = from_float<TS>(xn[it]);
     }
   }
+  copy_async_wait();
   __syncthreads();
 
   // both gate projections of the block: g[gate][b][j] = bias[j] + sum_k xc[b][k] w[k][j]  (external.py:224-233)
-  for (int o = threadIdx.x; o < 2 * bw; o += blockDim.x) {
-    const int gate = o / bw, j = o - gate * bw;
-    const TW* wp = ws + (size_t)gate * bw * bw + j;
-    const float bias = (gate ? ba : bx)[ch0 + j];
-    float2 acc[kDecTB / 2];  // batch rows in pairs: packed fp32x2 FMAs, same rounding as scalar ones
+  // A thread takes one output column for NB batch rows; narrow blocks have few columns, so their rows are dealt out too
+  // (all 16 rows to a thread left 192 of the 256 threads of a 32-wide block idle)
+  auto products = [&](auto nb_c) {
+    constexpr int NB = decltype(nb_c)::value;
+    for (int id = threadIdx.x; id < 2 * bw * (kDecTB / NB); id += blockDim.x) {
+      const int o = id % (2 * bw), r0 = id / (2 * bw) * NB;
+      const int gate = o / bw, j = o - gate * bw;
+      const TW* wp = ws + (size_t)gate * bw * bw + j;
+      const float bias = (gate ? ba : bx)[ch0 + j];
+      float2 acc[NB / 2];  // batch rows in pairs: packed fp32x2 FMAs, same rounding as scalar ones
 #pragma unroll
-    for (int b = 0; b < kDecTB / 2; ++b) acc[b] = f2(bias);
+      for (int b = 0; b < NB / 2; ++b) acc[b] = f2(bias);
 #pragma unroll 4
-    for (int k = 0; k < bw; ++k) {
-      const float2 wv = f2(to_float(wp[k * bw]));
-      const float4* xr = reinterpret_cast<const float4*>(xcT + k * kDecTB);
+      for (int k = 0; k < bw; ++k) {
+        const float2 wv = f2(to_float(wp[k * bw]));
+        const float4* xr = reinterpret_cast<const float4*>(xcT + k * kDecTB + r0);
 #pragma unroll
-      for (int q = 0; q < kDecTB / 4; ++q) {
-        const float4 xv = xr[q];
-        acc[2 * q] = fma2(make_float2(xv.x, xv.y), wv, acc[2 * q]);
-        acc[2 * q + 1] = fma2(make_float2(xv.z, xv.w), wv, acc[2 * q + 1]);
+        for (int q = 0; q < NB / 4; ++q) {
+          const float4 xv = xr[q];
+          acc[2 * q] = fma2(make_float2(xv.x, xv.y), wv, acc[2 * q]);
+          acc[2 * q + 1] = fma2(make_float2(xv.z, xv.w), wv, acc[2 * q + 1]);
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < NB / 2; ++b) {
+        g[((size_t)gate * kDecTB + r0 + 2 * b) * bw + j] = acc[b].x;
+        g[((size_t)gate * kDecTB + r0 + 2 * b + 1) * bw + j] = acc[b].y;
       }
     }
-#pragma unroll
-    for (int b = 0; b < kDecTB / 2; ++b) {
-      g[((size_t)gate * kDecTB + 2 * b) * bw + j] = acc[b].x;
-      g[((size_t)gate * kDecTB + 2 * b + 1) * bw + j] = acc[b].y;
-    }
-  }
+  };
+  if (bw <= 32) products(std::integral_constant<int, 4>{});
+  else if (bw <= 64) products(std::integral_constant<int, 8>{});
+  else products(std::integral_constant<int, 16>{});
   __syncthreads();
 
   // RG-LRU step (hawk/hawk.py:137-151,193-198) and the output gate gelu(y) * h (:134-135)
@@ -251,6 +258,25 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
   const int blk = blockIdx.x, b0 = blockIdx.y * TB, ch0 = blk * BW;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
+  {  // weights: rows of BW elements into rows of KP, 16 bytes at a time (global rows are 16-byte aligned: host check), in
+     // flight while the other inputs are and, in a chain of launches, while the kernel before this one finishes
+    constexpr int Q = BW / 8;
+    const bf* s0 = wx + (int64_t)blk * BW * BW;
+    const bf* s1 = wa + (int64_t)blk * BW * BW;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < BW * Q; i += 256) {
+      const int k = i / Q, q = i % Q;
+      copy_async16(ws + k * KP + q * 8, s0 + i * 8);
+      copy_async16(ws + (BW + k) * KP + q * 8, s1 + i * 8);
+    }
+  }
+  if (threadIdx.x < BW) {
+    const float l = lam[ch0 + threadIdx.x];
+    spc[threadIdx.x] = l > 20.f ? l : softplus_f(l);
+  }
+  pdl_wait();
+  pdl_trigger();
+
   // A thread owns 8 consecutive channels of one batch row (TB * BW / 8 <= 256 threads have work): every
   // global input arrives as 16-byte loads, all requested before anything waits.
   constexpr int VEC = 8, TPR = BW / VEC;  // threads per batch row
@@ -263,13 +289,13 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
     const int64_t bg = b0 + eb;
     const int ch = ch0 + ec;
     const bf* xr = xy + bg * ld_xy;
-    VecIO<bf, VEC>::load(xr + ch, xn);
-    VecIO<bf, VEC>::load(xr + R + ch, yv);
-    VecIO<TS, VEC>::load(state + bg * R + ch, sv);
+    load_dep8(xr + ch, xn);
+    load_dep8(xr + R + ch, yv);
+    load_dep8(state + bg * R + ch, sv);
     const TS* sp = conv_state + (bg * (W - 1)) * R + ch;
 #pragma unroll
     for (int j = 0; j < 3; ++j)
-      if (j < W - 1) VecIO<TS, VEC>::load(sp + (int64_t)j * R, win[j]);
+      if (j < W - 1) load_dep8(sp + (int64_t)j * R, win[j]);
     float wv[VEC];
     VecIO<float, VEC>::load(cb + ch, cacc);
     VecIO<float, VEC>::load(cw + (int64_t)(W - 1) * R + ch, wv);
@@ -284,21 +310,6 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
       }
     }
   }
-  {  // weights: rows of BW elements into rows of KP, 16 bytes at a time (global rows are 16-byte aligned: host check)
-    constexpr int Q = BW / 8;
-    const uint4* s0 = reinterpret_cast<const uint4*>(wx + (int64_t)blk * BW * BW);
-    const uint4* s1 = reinterpret_cast<const uint4*>(wa + (int64_t)blk * BW * BW);
-#pragma unroll 4
-    for (int i = threadIdx.x; i < BW * Q; i += 256) {
-      const int k = i / Q, q = i % Q;
-      *reinterpret_cast<uint4*>(ws + k * KP + q * 8) = __ldg(s0 + i);
-      *reinterpret_cast<uint4*>(ws + (BW + k) * KP + q * 8) = __ldg(s1 + i);
-    }
-  }
-  if (threadIdx.x < BW) {
-    const float l = lam[ch0 + threadIdx.x];
-    spc[threadIdx.x] = l > 20.f ? l : softplus_f(l);
-  }
   // conv outputs (rounded to bf16) to shared memory, and the cache roll (hawk/hawk.py:168-179, hawk/cache.py:37-43)
   if (has) VecIO<bf, VEC>::store(xcb + eb * KP + ec, cacc);  // rows past the batch hold zeros
   if (ok) {
@@ -308,6 +319,7 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
       if (j < W - 1) VecIO<TS, VEC>::store(sp + (int64_t)(j - 1) * R, win[j]);
     if (W > 1) VecIO<TS, VEC>::store(sp + (int64_t)(W - 2) * R, xn);
   }
+  copy_async_wait();
   __syncthreads();
 
   // both gate projections: g[gate][b][j] = bias[j] + sum_k xc[b][k] w[gate][k][j]  (external.py:224-233)
@@ -443,7 +455,7 @@ namespace hawk {
 template <typename T, typename TS, typename TW>
 static int block_step_launch(const void* xy, int64_t ld_xy, void* conv_state, const float* cw, const float* cb,
                              const void* wx, const void* wa, const float* bx, const float* ba, const float* lam,
-                             void* state, void* out, int B, int R, int bw, int W, cudaStream_t st) {
+                             void* state, void* out, int B, int R, int bw, int W, bool pdl, cudaStream_t st) {
   dim3 grid((unsigned)(R / bw), (unsigned)((B + kDecTB - 1) / kDecTB));
   if constexpr (std::is_same<T, __nv_bfloat16>::value && std::is_same<TW, __nv_bfloat16>::value) {
     const bool rows16 = aligned(wx, 16) && aligned(wa, 16) && aligned(bx, 8) && aligned(ba, 8) && aligned(xy, 16) &&
@@ -459,10 +471,10 @@ static int block_step_launch(const void* xy, int64_t ld_xy, void* conv_state, co
       (void)cudaGetLastError();                                                                                      \
       return HAWK_ERR_LAUNCH;                                                                                        \
     }                                                                                                                \
-    kmma<<<grid, 256, smem_mma, st>>>(static_cast<const __nv_bfloat16*>(xy), ld_xy, static_cast<TS*>(conv_state), cw, \
-                                      cb, static_cast<const __nv_bfloat16*>(wx), static_cast<const __nv_bfloat16*>(wa), \
-                                      bx, ba, lam, static_cast<TS*>(state), static_cast<__nv_bfloat16*>(out), B, R, W); \
-    return launch_status();                                                                                          \
+    return launch_kernel(kmma, grid, dim3(256), (size_t)smem_mma, st, pdl, 1, static_cast<const __nv_bfloat16*>(xy), ld_xy, \
+                         static_cast<TS*>(conv_state), cw, cb, static_cast<const __nv_bfloat16*>(wx),                 \
+                         static_cast<const __nv_bfloat16*>(wa), bx, ba, lam, static_cast<TS*>(state),                 \
+                         static_cast<__nv_bfloat16*>(out), B, R, W);                                                  \
   } while (0)
       if (bw == 128) HAWK_DEC_MMA(128);
       if (bw == 64) HAWK_DEC_MMA(64);
@@ -478,10 +490,26 @@ static int block_step_launch(const void* xy, int64_t ld_xy, void* conv_state, co
     (void)cudaGetLastError();
     return HAWK_ERR_LAUNCH;
   }
-  kern<<<grid, 256, smem, st>>>(
-      static_cast<const T*>(xy), ld_xy, static_cast<TS*>(conv_state), cw, cb, static_cast<const TW*>(wx),
-      static_cast<const TW*>(wa), bx, ba, lam, static_cast<TS*>(state), static_cast<T*>(out), B, R, bw, W);
-  return launch_status();
+  return launch_kernel(kern, grid, dim3(256), smem, st, pdl, 1, static_cast<const T*>(xy), ld_xy, static_cast<TS*>(conv_state),
+                       cw, cb, static_cast<const TW*>(wx), static_cast<const TW*>(wa), bx, ba, lam, static_cast<TS*>(state),
+                       static_cast<T*>(out), B, R, bw, W);
+}
+
+int block_step(const void* xy, int64_t ld_xy, void* conv_state, const float* cw, const float* cb, const void* wx, const void* wa,
+               const float* bx, const float* ba, const float* lam, void* state, void* out, int B, int R, int bw, int W, int dtype,
+               int state_dtype, int weight_dtype, bool pdl, cudaStream_t st) {
+#define HAWK_DEC_BLOCK(T, TS, TW)                                                                                    \
+  return block_step_launch<T, TS, TW>(xy, ld_xy, conv_state, cw, cb, wx, wa, bx, ba, lam, state, out, B, R, bw, W, pdl, st)
+  const bool xb = dtype == HAWK_BF16, sb = state_dtype == HAWK_BF16, wb = weight_dtype == HAWK_BF16;
+  if (xb && sb && wb) HAWK_DEC_BLOCK(bf, bf, bf);
+  if (xb && sb) HAWK_DEC_BLOCK(bf, bf, float);
+  if (xb && wb) HAWK_DEC_BLOCK(bf, float, bf);
+  if (xb) HAWK_DEC_BLOCK(bf, float, float);
+  if (sb && wb) HAWK_DEC_BLOCK(float, bf, bf);
+  if (sb) HAWK_DEC_BLOCK(float, bf, float);
+  if (wb) HAWK_DEC_BLOCK(float, float, bf);
+  HAWK_DEC_BLOCK(float, float, float);
+#undef HAWK_DEC_BLOCK
 }
 }  // namespace hawk
 
@@ -497,18 +525,6 @@ extern "C" int hawk_decode_block_step(const void* xy, int64_t xy_row_stride, voi
                HAWK_ERR_SHAPE);
   HAWK_REQUIRE(W >= 1 && W <= 4 && block_width <= 128, HAWK_ERR_UNSUPPORTED);  // weights staged in shared memory
   HAWK_REQUIRE((int64_t)((B + kDecTB - 1) / kDecTB) <= 65535, HAWK_ERR_SHAPE);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define HAWK_DEC_BLOCK(T, TS, TW)                                                                                  \
-  return block_step_launch<T, TS, TW>(xy, xy_row_stride, conv_state, conv_w, conv_b, wx, wa, bx, ba, lam, state, out, \
-                                      B, R, block_width, W, st)
-  const bool xb = dtype == HAWK_BF16, sb = state_dtype == HAWK_BF16, wb = weight_dtype == HAWK_BF16;
-  if (xb && sb && wb) HAWK_DEC_BLOCK(bf, bf, bf);
-  if (xb && sb) HAWK_DEC_BLOCK(bf, bf, float);
-  if (xb && wb) HAWK_DEC_BLOCK(bf, float, bf);
-  if (xb) HAWK_DEC_BLOCK(bf, float, float);
-  if (sb && wb) HAWK_DEC_BLOCK(float, bf, bf);
-  if (sb) HAWK_DEC_BLOCK(float, bf, float);
-  if (wb) HAWK_DEC_BLOCK(float, float, bf);
-  HAWK_DEC_BLOCK(float, float, float);
-#undef HAWK_DEC_BLOCK
+  return block_step(xy, xy_row_stride, conv_state, conv_w, conv_b, wx, wa, bx, ba, lam, state, out, B, R, block_width, W, dtype,
+                    state_dtype, weight_dtype, false, static_cast<cudaStream_t>(stream));
 }

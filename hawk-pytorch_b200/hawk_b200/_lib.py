@@ -17,6 +17,17 @@ HAWK_BF16 = 1
 ABI_VERSION = 5
 
 _P = c_void_p
+
+class DecodeLayerArgs(ctypes.Structure):
+    """hawk_decode_layer_args, field by field."""
+    _fields_ = ([(n, _P) for n in ("residual", "pending", "norm1_w", "w_xy", "conv_w", "conv_b", "wx", "wa", "bx", "ba", "lam",
+                                   "w_res", "norm2_w", "w_gu", "w_down", "conv_state", "state", "out_residual", "out_pending",
+                                   "workspace", "status")]
+                + [("workspace_bytes", c_size_t), ("eps1", c_float), ("eps2", c_float)]
+                + [(n, c_int) for n in ("B", "H", "R", "I", "block_width", "W", "res_dtype", "state_dtype", "gate_dtype",
+                                        "xy_dtype", "resid_dtype", "gu_dtype", "down_dtype", "follows_layer")])
+
+
 # name -> (restype, argtypes); mirrors include/hawk_b200.h one to one
 SIGNATURES = {
     "hawk_version": (c_int, []),
@@ -40,6 +51,9 @@ SIGNATURES = {
     "hawk_decode_conv_step": (c_int, [_P, c_int64, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P]),
     "hawk_decode_rglru_step": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "hawk_decode_block_step": (c_int, [_P, c_int64] + [_P] * 10 + [c_int] * 7 + [_P]),
+    "hawk_decode_layer_workspace_bytes": (c_size_t, [c_int] * 5),
+    "hawk_decode_layer": (c_int, [ctypes.POINTER(DecodeLayerArgs), _P]),
+    "hawk_decode_norm_linear": (c_int, [_P, _P, _P, c_float, _P, _P, _P, c_size_t] + [c_int] * 6 + [_P, _P]),
     "hawk_adamw_step": (c_int, [_P, _P, _P, _P, _P, c_int64, c_float, c_float, c_float, c_float, c_float, c_int64, _P]),
     "hawk_cast_f32_bf16": (c_int, [_P, _P, c_int64, _P]),
     "hawk_gelu_mul_fwd": (c_int, [_P, c_int64, _P, c_int64, _P, c_int64, c_int64, c_int, c_int, _P]),

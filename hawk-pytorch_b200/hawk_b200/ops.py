@@ -594,6 +594,79 @@ def _(x, gx, ga, lam, state):
     return torch.empty_like(x)
 
 
+def _dense16(t: torch.Tensor) -> torch.Tensor:
+    """t contiguous at a 16-byte aligned address."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+@torch.library.custom_op("hawk_b200::decode_layer", mutates_args=("conv_state", "state"))
+def decode_layer(residual: torch.Tensor, pending: Optional[torch.Tensor], norm1: torch.Tensor, eps1: float, w_xy: torch.Tensor,
+                 conv_w: torch.Tensor, conv_b: torch.Tensor, wx: torch.Tensor, wa: torch.Tensor, bx: torch.Tensor,
+                 ba: torch.Tensor, lam: torch.Tensor, w_res: torch.Tensor, norm2: torch.Tensor, eps2: float, w_gu: torch.Tensor,
+                 w_down: torch.Tensor, conv_state: torch.Tensor, state: torch.Tensor, follows_layer: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    """One cached token through a whole layer: (residual, pending) -> (residual, pending), [.., H] for up to 256 rows; norms,
+    taps, biases and Lambda in fp32, projection weights fp32 (rounded to bf16 as they are read) or bf16, activations bf16.  follows_layer: nothing has run on the stream since
+    the call for the layer before (its kernels and this one's may then overlap further)."""
+    lib = _lib.load()
+    H = residual.shape[-1]
+    B, R, (nb, bw, _), I = residual.numel() // H, lam.numel(), wx.shape, w_down.shape[1]
+    assert w_xy.shape == (2 * R, H) and w_res.shape == (H, R) and w_gu.shape == (2 * I, H) and w_down.shape == (H, I)
+    assert nb * bw == R and wx.dtype == wa.dtype and (pending is None or pending.dtype == torch.bfloat16)
+    assert conv_state.is_contiguous() and state.is_contiguous() and state.numel() == B * R and conv_state.dtype == state.dtype
+    residual = _dense16(residual)
+    pending = None if pending is None else _dense16(pending)
+    keep = [_dense16(t) for t in (norm1, w_xy, conv_w, conv_b, wx, wa, bx, ba, lam, w_res, norm2, w_gu, w_down)]
+    n1, wxy, cw, cb, kx, ka, vx, va, lm, wr, n2, wg, wd = keep
+    out_res = torch.empty_like(residual)
+    out_pending = torch.empty(residual.shape, dtype=torch.bfloat16, device=residual.device)
+    ws = torch.empty(lib.hawk_decode_layer_workspace_bytes(B, H, R, I, _dt(residual)), dtype=torch.uint8, device=residual.device)
+    args = _lib.DecodeLayerArgs(
+        residual=_ptr(residual), pending=_ptr(pending), norm1_w=_ptr(n1), w_xy=_ptr(wxy), conv_w=_ptr(cw), conv_b=_ptr(cb),
+        wx=_ptr(kx), wa=_ptr(ka), bx=_ptr(vx), ba=_ptr(va), lam=_ptr(lm), w_res=_ptr(wr), norm2_w=_ptr(n2), w_gu=_ptr(wg),
+        w_down=_ptr(wd), conv_state=_ptr(conv_state), state=_ptr(state), out_residual=_ptr(out_res),
+        out_pending=_ptr(out_pending), workspace=_ptr(ws), status=_ptr(_status_word(residual.device)), workspace_bytes=ws.numel(),
+        eps1=eps1, eps2=eps2, B=B, H=H, R=R, I=I, block_width=bw, W=conv_w.shape[0], res_dtype=_dt(residual),
+        state_dtype=_dt(state), gate_dtype=_dt(wx), xy_dtype=_dt(w_xy), resid_dtype=_dt(w_res), gu_dtype=_dt(w_gu),
+        down_dtype=_dt(w_down), follows_layer=int(follows_layer))
+    with _on(residual, "decode_layer", 5 if B <= 8 or (B <= 16 and max(H, R) <= 512) else 7):
+        _lib.check(lib.hawk_decode_layer(args, _stream(residual)), "hawk_decode_layer")
+    return out_res, out_pending
+
+
+@decode_layer.register_fake
+def _(residual, pending, norm1, eps1, w_xy, conv_w, conv_b, wx, wa, bx, ba, lam, w_res, norm2, eps2, w_gu, w_down, conv_state,
+      state, follows_layer):
+    return (torch.empty_like(residual, memory_format=torch.contiguous_format),
+            residual.new_empty(residual.shape, dtype=torch.bfloat16))
+
+
+@torch.library.custom_op("hawk_b200::decode_norm_linear", mutates_args=())
+def decode_norm_linear(residual: torch.Tensor, pending: Optional[torch.Tensor], norm: torch.Tensor, eps: float,
+                       weight: torch.Tensor, follows_layer: bool) -> torch.Tensor:
+    """bf16 rms_norm(residual + pending) @ weight^T for up to 256 rows [.., H] (the final norm and the head of a cached token);
+    `weight` [N, H] fp32 (rounded to bf16 as it is read) or bf16; follows_layer as in decode_layer."""
+    lib = _lib.load()
+    H, N = residual.shape[-1], weight.shape[0]
+    B = residual.numel() // H
+    assert weight.shape == (N, H) and (pending is None or pending.dtype == torch.bfloat16)
+    residual, norm, weight = _dense16(residual), _dense16(norm), _dense16(weight)
+    pending = None if pending is None else _dense16(pending)
+    out = torch.empty(*residual.shape[:-1], N, dtype=torch.bfloat16, device=residual.device)
+    ws = torch.empty(B * H * 2 + B * H * residual.element_size() + 512, dtype=torch.uint8, device=residual.device)
+    with _on(residual, "decode_norm_linear", 1 if B <= 8 or (B <= 16 and H <= 512) else 2):
+        _lib.check(lib.hawk_decode_norm_linear(_ptr(residual), _ptr(pending), _ptr(norm), eps, _ptr(weight), _ptr(out), _ptr(ws),
+                                               ws.numel(), B, H, N, _dt(residual), _dt(weight), int(follows_layer),
+                                               _ptr(_status_word(residual.device)), _stream(residual)),
+                   "hawk_decode_norm_linear")
+    return out
+
+
+@decode_norm_linear.register_fake
+def _(residual, pending, norm, eps, weight, follows_layer):
+    return residual.new_empty(*residual.shape[:-1], weight.shape[0], dtype=torch.bfloat16)
+
+
 # ---------------------------------------------------------------------------------------------
 # fused linear + cross-entropy
 # ---------------------------------------------------------------------------------------------

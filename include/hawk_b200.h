@@ -188,6 +188,41 @@ int hawk_decode_block_step(const void* xy, int64_t xy_row_stride, void* conv_sta
                            const float* lam, void* state, void* out, int B, int R, int block_width, int W,
                            int dtype, int state_dtype, int weight_dtype, void* stream);
 
+/* One cached token of B <= 256 rows through a whole layer (hawk/hawk.py:206-236) as one chain of overlapping launches:
+ *   residual += pending; xy = norm1(residual) . w_xy^T; branch = hawk_decode_block_step(xy); residual += branch . w_res^T;
+ *   out_residual = residual; out_pending = (gelu(gate) * up) . w_down^T with [gate | up] = norm2(residual) . w_gu^T.
+ * Activations, projections' results and out_pending are bf16; residual and out_residual [B,H] have res_dtype; pending may be
+ * NULL.  Projection weights are row-major [out, in], fp32 (rounded to bf16 as they are read) or bf16, each
+ * with a type of its own; gate weights and the caches as in hawk_decode_block_step.  H, R, I multiples of 8, H <= 8192; all
+ * pointers 16-byte aligned; nothing may be written elsewhere while the call's kernels run;
+ * follows_layer: the kernel before this call on the stream is that of another hawk_decode_layer, so that w_xy may be read
+ * before it has ended.  Waits are bounded: `status` as in
+ * hawk_linear_ce_fwd_bwd, and the results of a launch that gave up are NaN. */
+typedef struct hawk_decode_layer_args {
+  const void *residual, *pending;
+  const float* norm1_w;
+  const void* w_xy;
+  const float *conv_w, *conv_b;
+  const void *wx, *wa;
+  const float *bx, *ba, *lam;
+  const void* w_res;
+  const float* norm2_w;
+  const void *w_gu, *w_down;
+  void *conv_state, *state, *out_residual, *out_pending, *workspace;
+  int* status;
+  size_t workspace_bytes;
+  float eps1, eps2;
+  int B, H, R, I, block_width, W;
+  int res_dtype, state_dtype, gate_dtype, xy_dtype, resid_dtype, gu_dtype, down_dtype, follows_layer;
+} hawk_decode_layer_args;
+size_t hawk_decode_layer_workspace_bytes(int B, int H, int R, int I, int res_dtype);
+int hawk_decode_layer(const hawk_decode_layer_args* args, void* stream);
+/* out [B,N] bf16 = norm(residual + pending) . w^T for B <= 256 (the final norm and the head, hawk/hawk.py:300-303).  N a multiple
+ * of 8; workspace: B*H*2 bytes, and B*H elements of res_dtype with `pending`, each rounded up to 256. */
+int hawk_decode_norm_linear(const void* residual, const void* pending, const float* norm_w, float eps, const void* w, void* out,
+                            void* workspace, size_t workspace_bytes, int B, int H, int N, int res_dtype, int w_dtype,
+                            int follows_layer, int* status, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Fused linear + cross-entropy.  Replaces CrossEntropyLoopedFused.forward
  * (hawk/fused_cross_entropy.py:13-64): mean cross-entropy of act @ weight^T against labels, and

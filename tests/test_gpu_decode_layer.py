@@ -1,0 +1,91 @@
+"""The chained decode kernels: a projection at the edges of its tiles, splits and token counts, and a whole cached token
+against the same modules called one by one."""
+import pytest
+import torch
+
+import hawk_b200.ops as ops
+from conftest import rel_l2
+from hawk_b200.generate import GraphedDecoder
+from hawk_b200.model import HawkConfig, HawkModel
+
+pytestmark = pytest.mark.gpu
+
+
+# rows: one, a full and a ragged group of 8 and of 16 (the most that decode_rows_kernel takes), the fewest of the other kernel,
+# more than one of its reduction passes (two of 128), the most
+# (H, N): one K block and one tile; K not a multiple of 64 with a ragged tile; every K split up to 8; more tiles than SMs
+@pytest.mark.parametrize("rows", [1, 8, 11, 16, 17, 129, 256])
+@pytest.mark.parametrize("H,N", [(64, 8), (72, 136), (520, 200), (1536, 768), (2048, 20000)])
+@pytest.mark.parametrize("wdt,rdt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+def test_norm_linear(rows, H, N, wdt, rdt):
+    torch.manual_seed(rows + H + N)
+    res = torch.randn(rows, 1, H, device="cuda").to(rdt)
+    pend = torch.randn(rows, 1, H, device="cuda").bfloat16()
+    norm = torch.rand(H, device="cuda") + 0.5
+    w = (torch.randn(N, H, device="cuda") / H**0.5).to(wdt)
+    for p in (None, pend):
+        out = ops.decode_norm_linear(res, p, norm, 1e-6, w, False)
+        s = res if p is None else (res.float() + p.float()).to(rdt)
+        s = s.double()
+        x = (s * torch.rsqrt((s * s).mean(-1, keepdim=True) + 1e-6) * norm.double()).float().bfloat16().double()
+        ref = x @ w.bfloat16().double().t()
+        # the result is one rounding to bf16 (2^-9 relative at most); x's own roundings can differ in ties only
+        assert out.shape == (rows, 1, N) and rel_l2(out, ref) < 3e-3
+    ops.check_device_status()
+
+
+def _model(vocab, hidden, inter, layers, blocks):
+    with torch.device("cuda"):
+        model = HawkModel(HawkConfig(vocab, hidden, inter, layers, hidden, blocks, 4), use_cache=True)
+    with torch.no_grad():
+        for p in model.parameters():
+            if p.dim() == 2 and float(p.abs().max()) == 0.0:
+                p.normal_(0.0, p.shape[1] ** -0.5)
+    return model
+
+
+CASES = [(64, 72, 4, b, half) for b in (1, 13, 19, 32) for half in (True, False)]
+CASES += [(256, 768, 16, b, half) for b in (1, 13, 19, 32) for half in (True, False)]
+CASES += [(2048, 6144, 16, b, True) for b in (1, 8)] + [(2048, 6144, 16, b, False) for b in (1, 13, 64)]
+
+
+@pytest.mark.parametrize("hidden,inter,blocks,batch,half", CASES)
+def test_cached_token_against_modules(hidden, inter, blocks, batch, half):
+    torch.manual_seed(hidden + batch)
+    model = _model(1000, hidden, inter, 2, blocks)
+    if half:
+        model = model.bfloat16()
+    dec = GraphedDecoder(model, batch, autocast=not half, use_graph=False)
+    ids = torch.randint(0, 1000, (batch, 6), device="cuda")
+    outs = []
+    for hooked in (False, True):
+        # a hook on a module keeps its layer (and the head) on the module-by-module path
+        handles = [m.register_forward_hook(lambda *_: None) for m in model.modules() if isinstance(m, torch.nn.Linear)] if hooked else []
+        dec.prefill(ids[:, :4])
+        ops.LOG.reset()
+        logits = [dec.step(ids[:, t:t + 1]) for t in (4, 5)]
+        counts = dict(ops.LOG.counts)
+        ops.LOG.reset(enabled=False)
+        assert ("decode_layer" in counts) == (not hooked) and ("decode_norm_linear" in counts) == (not hooked)
+        outs.append((logits, [(c.recc_state.clone(), c.conv_state.clone()) for c in dec.caches]))
+        for h in handles:
+            h.remove()
+    (la, ca), (lb, cb) = outs
+    # both are bf16 computations that differ in the order of fp32 sums: a few bf16 roundings (2^-9 each) of two layers
+    for a, b in zip(la, lb):
+        assert a.dtype == b.dtype and a.shape == b.shape and rel_l2(a, b) < 2e-2
+    for (ra, ka), (rb, kb) in zip(ca, cb):
+        assert rel_l2(ra, rb) < 2e-2 and rel_l2(ka, kb) < 2e-2
+    ops.check_device_status()
+
+
+def test_graph_replay_equals_direct_calls():
+    torch.manual_seed(0)
+    model = _model(1000, 256, 512, 3, 16).bfloat16()
+    ids = torch.randint(0, 1000, (5, 12), device="cuda")
+    res = []
+    for graph in (False, True):
+        dec = GraphedDecoder(model, 5, autocast=False, use_graph=graph)
+        dec.prefill(ids[:, :4])
+        res.append(torch.cat([dec.step(ids[:, t:t + 1]).clone() for t in range(4, 12)], 1))
+    assert torch.equal(res[0], res[1])  # the same kernels in the same order of sums
