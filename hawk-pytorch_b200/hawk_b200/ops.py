@@ -17,6 +17,7 @@ must live on a CUDA device and the library must have been built.
 """
 from __future__ import annotations
 
+import inspect
 import math
 from typing import Optional, Tuple
 
@@ -39,7 +40,7 @@ def _dt(t: torch.Tensor) -> int:
 def _stream(t: torch.Tensor) -> int:
     if not t.is_cuda:
         raise RuntimeError("hawk_b200: tensors must be on a CUDA device (there is no CPU path)")
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -91,7 +92,7 @@ class _on:
         self.start = None
 
     def __enter__(self):
-        cur = torch.cuda.current_device()
+        cur = torch._C._cuda_getDevice()
         if self.idx is not None and self.idx != cur:
             self.prev = cur
             torch.cuda.set_device(self.idx)
@@ -112,6 +113,76 @@ class _on:
 
 
 # ---------------------------------------------------------------------------------------------
+# operators
+# ---------------------------------------------------------------------------------------------
+def _plain_call(args) -> Optional[bool]:
+    """None where a call belongs to the dispatcher: tracing, transforms, forward-mode derivatives, function and dispatch modes,
+    tensor subclasses, devices other than CUDA.  Otherwise whether autograd has to record it."""
+    C = torch._C
+    if (torch.compiler.is_compiling() or C._len_torch_dispatch_stack() or C._len_torch_function_stack()
+            or C._functorch.peek_interpreter_stack() is not None or C._get_tracing_state() is not None
+            or torch.autograd.forward_ad._current_level >= 0):
+        return None
+    grad = False
+    for a in args:
+        if isinstance(a, torch.Tensor):
+            if (type(a) is not torch.Tensor and type(a) is not nn.Parameter) or not a.is_cuda:
+                return None
+            grad = grad or a.requires_grad
+    return grad and torch.is_grad_enabled()
+
+
+class _Operator:
+    """A torch.library operator whose ordinary eager calls run its Python function directly, with autograd through one
+    torch.autograd.Function.  The dispatcher's way through a Python operator costs 40 to 60 us of host time per call, more
+    than most of these kernels take on the GPU: the 24-layer prefill of 3108 tokens (169 such calls) took 12.5 ms against
+    7.8 ms of kernels, a training step of 1551 tokens 7.4 ms against 1.3.  Everything else (see _plain_call) takes it."""
+
+    def __init__(self, name, mutates_args, fn):
+        self.op = torch.library.custom_op(name, mutates_args=mutates_args)(fn)
+        self.fn, self.function = fn, None
+        names = list(inspect.signature(fn).parameters)
+        self.nargs = len(names)
+        self.mutated = [names.index(m) for m in mutates_args]
+        self.__doc__, self.__name__ = fn.__doc__, fn.__name__
+
+    def register_fake(self, fn):
+        return self.op.register_fake(fn)
+
+    def register_autograd(self, backward, *, setup_context):
+        self.op.register_autograd(backward, setup_context=setup_context)
+        fn = self.fn
+
+        class Function(torch.autograd.Function):
+            @staticmethod
+            def forward(ctx, *args):
+                out = fn(*args)
+                setup_context(ctx, args, out)
+                return out
+
+        Function.backward = staticmethod(backward)
+        Function.__name__ = Function.__qualname__ = fn.__name__
+        self.function = Function
+
+    def __call__(self, *args, **kwargs):
+        if not kwargs and len(args) == self.nargs:
+            record = _plain_call(args)
+            if record is False:
+                out = self.fn(*args)
+                for i in self.mutated:  # what the dispatcher does for a mutated argument
+                    if not args[i].is_inference():
+                        torch.autograd.graph.increment_version(args[i])
+                return out
+            if record and self.function is not None:
+                return self.function.apply(*args)
+        return self.op(*args, **kwargs)
+
+
+def _operator(name, mutates_args):
+    return lambda fn: _Operator(name, mutates_args, fn)
+
+
+# ---------------------------------------------------------------------------------------------
 # RG-LRU scan
 # ---------------------------------------------------------------------------------------------
 # bytes each entry point must move per [B,T,D] element with bf16 storage (its HBM roofline), and the
@@ -128,7 +199,7 @@ def _split_view_ok(v, T):
     return v.shape[0] == 1 or v.stride(0) == T * v.stride(1)
 
 
-@torch.library.custom_op("hawk_b200::scan_fwd", mutates_args=())
+@_operator("hawk_b200::scan_fwd", mutates_args=())
 def scan_fwd(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Tensor,
              h0: Optional[torch.Tensor] = None, gate_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     lib = _lib.load()
@@ -159,7 +230,7 @@ def _(x, gx, ga, lam, h0=None, gate_bias=None):
     return torch.empty_like(x, memory_format=torch.contiguous_format)
 
 
-@torch.library.custom_op("hawk_b200::scan_bwd", mutates_args=())
+@_operator("hawk_b200::scan_bwd", mutates_args=())
 def scan_bwd(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Tensor, h0: Optional[torch.Tensor],
              gate_bias: Optional[torch.Tensor], h: torch.Tensor, go: torch.Tensor
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
@@ -270,7 +341,7 @@ def _conv_view(x: torch.Tensor) -> torch.Tensor:
 
 
 # ---- the scan with the block's epilogue out = gelu(y) * h fused in (hawk/hawk.py:134-135,201) ----
-@torch.library.custom_op("hawk_b200::scan_gelu_fwd", mutates_args=())
+@_operator("hawk_b200::scan_gelu_fwd", mutates_args=())
 def scan_gelu_fwd(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Tensor,
                   gate_bias: Optional[torch.Tensor], y: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """(h, gelu(y) * h); y [B,T,D] may be a row-strided view (the y half of the input projection)."""
@@ -305,7 +376,7 @@ def _(x, gx, ga, lam, gate_bias, y):
     return e(), e()
 
 
-@torch.library.custom_op("hawk_b200::scan_gelu_bwd_into", mutates_args=("dy_out",))
+@_operator("hawk_b200::scan_gelu_bwd_into", mutates_args=("dy_out",))
 def scan_gelu_bwd_into(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Tensor,
                        gate_bias: Optional[torch.Tensor], h: torch.Tensor, y: torch.Tensor, dout: torch.Tensor,
                        dy_out: torch.Tensor
@@ -392,7 +463,7 @@ def fused_scan_gelu(x, x_rg_lru, a_rg_lru, a_param, y, *, gate_bias=None):
 # ---------------------------------------------------------------------------------------------
 
 
-@torch.library.custom_op("hawk_b200::conv1d_fwd", mutates_args=())
+@_operator("hawk_b200::conv1d_fwd", mutates_args=())
 def conv1d_fwd(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     lib = _lib.load()
     B, T, D = x.shape
@@ -411,7 +482,7 @@ def _(x, w, b, out_dtype):
     return x.new_empty(x.shape, dtype=out_dtype)
 
 
-@torch.library.custom_op("hawk_b200::conv1d_bwd", mutates_args=())
+@_operator("hawk_b200::conv1d_bwd", mutates_args=())
 def conv1d_bwd(go: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     lib = _lib.load()
     B, T, D = x.shape
@@ -452,7 +523,7 @@ def _conv_backward(ctx, go):
 conv1d_fwd.register_autograd(_conv_backward, setup_context=_conv_setup)
 
 
-@torch.library.custom_op("hawk_b200::conv1d_bwd_into", mutates_args=("dx_out",))
+@_operator("hawk_b200::conv1d_bwd_into", mutates_args=("dx_out",))
 def conv1d_bwd_into(go: torch.Tensor, x: torch.Tensor, w: torch.Tensor,
                     dx_out: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """conv1d_bwd with the input gradient written into `dx_out`, a [B,T,D] view that may be row-strided
@@ -521,7 +592,7 @@ class Conv1D(nn.Module):
 # ---------------------------------------------------------------------------------------------
 # cached decode step
 # ---------------------------------------------------------------------------------------------
-@torch.library.custom_op("hawk_b200::decode_conv_step", mutates_args=("conv_state",))
+@_operator("hawk_b200::decode_conv_step", mutates_args=("conv_state",))
 def decode_conv_step(x_new: torch.Tensor, conv_state: torch.Tensor, w: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """x_new [B,D] (row-strided ok), conv_state [B,W-1,D] contiguous, rolled in place. Returns y [B,D]."""
     lib = _lib.load()
@@ -542,7 +613,7 @@ def _(x_new, conv_state, w, b):
     return x_new.new_empty(x_new.shape)
 
 
-@torch.library.custom_op("hawk_b200::decode_block_step", mutates_args=("conv_state", "state"))
+@_operator("hawk_b200::decode_block_step", mutates_args=("conv_state", "state"))
 def decode_block_step(xy: torch.Tensor, conv_state: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor,
                       wx: torch.Tensor, wa: torch.Tensor, bx: torch.Tensor, ba: torch.Tensor, lam: torch.Tensor,
                       state: torch.Tensor) -> torch.Tensor:
@@ -573,7 +644,7 @@ def _(xy, conv_state, conv_w, conv_b, wx, wa, bx, ba, lam, state):
     return xy.new_empty(xy.shape[0], xy.shape[1] // 2)
 
 
-@torch.library.custom_op("hawk_b200::decode_rglru_step", mutates_args=("state",))
+@_operator("hawk_b200::decode_rglru_step", mutates_args=("state",))
 def decode_rglru_step(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Tensor,
                       state: torch.Tensor) -> torch.Tensor:
     """One recurrence step on [B,D]; `state` is overwritten with h; returns h in x's dtype."""
@@ -600,7 +671,7 @@ def _dense16(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-@torch.library.custom_op("hawk_b200::decode_layer", mutates_args=("conv_state", "state"))
+@_operator("hawk_b200::decode_layer", mutates_args=("conv_state", "state"))
 def decode_layer(residual: torch.Tensor, pending: Optional[torch.Tensor], norm1: torch.Tensor, eps1: float, w_xy: torch.Tensor,
                  conv_w: torch.Tensor, conv_b: torch.Tensor, wx: torch.Tensor, wa: torch.Tensor, bx: torch.Tensor,
                  ba: torch.Tensor, lam: torch.Tensor, w_res: torch.Tensor, norm2: torch.Tensor, eps2: float, w_gu: torch.Tensor,
@@ -641,7 +712,7 @@ def _(residual, pending, norm1, eps1, w_xy, conv_w, conv_b, wx, wa, bx, ba, lam,
             residual.new_empty(residual.shape, dtype=torch.bfloat16))
 
 
-@torch.library.custom_op("hawk_b200::decode_norm_linear", mutates_args=())
+@_operator("hawk_b200::decode_norm_linear", mutates_args=())
 def decode_norm_linear(residual: torch.Tensor, pending: Optional[torch.Tensor], norm: torch.Tensor, eps: float,
                        weight: torch.Tensor, follows_layer: bool) -> torch.Tensor:
     """bf16 rms_norm(residual + pending) @ weight^T for up to 256 rows [.., H] (the final norm and the head of a cached token);
@@ -691,7 +762,7 @@ def check_device_status(device=None) -> None:
             raise RuntimeError("hawk_b200: a tcgen05 GEMM abandoned a bounded mbarrier wait; results are invalid")
 
 
-@torch.library.custom_op("hawk_b200::linear_ce", mutates_args=())
+@_operator("hawk_b200::linear_ce", mutates_args=())
 def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """(loss [], dweight [V,H] fp32, dact [N,H] fp32) of mean CE(act @ weight^T, labels)."""
     lib = _lib.load()
@@ -725,7 +796,7 @@ linear_ce.register_autograd(
                                                setattr(ctx, "dtypes", (inputs[0].dtype, inputs[1].dtype)))[0])
 
 
-@torch.library.custom_op("hawk_b200::linear_ce_fwd", mutates_args=())
+@_operator("hawk_b200::linear_ce_fwd", mutates_args=())
 def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
                   want_grad: bool) -> Tuple[torch.Tensor, torch.Tensor]:
     """(loss [], saved): mean CE(act @ weight^T, labels) and, with want_grad, what linear_ce_bwd needs."""
@@ -757,7 +828,7 @@ def _(weight, act, labels, want_grad):
     return act.new_empty((), dtype=torch.float32), act.new_empty(n, dtype=torch.uint8)
 
 
-@torch.library.custom_op("hawk_b200::linear_ce_bwd", mutates_args=())
+@_operator("hawk_b200::linear_ce_bwd", mutates_args=())
 def linear_ce_bwd(weight: torch.Tensor, act: torch.Tensor, saved: torch.Tensor, grad_loss: torch.Tensor, want_dw: bool,
                   want_da: bool) -> Tuple[torch.Tensor, torch.Tensor]:
     """(d weight, d act) in the operands' dtypes, times grad_loss (empty where not wanted)."""
@@ -849,7 +920,7 @@ def _as_rows(t: torch.Tensor):
     return t, M, ld
 
 
-@torch.library.custom_op("hawk_b200::gelu_mul_fwd", mutates_args=())
+@_operator("hawk_b200::gelu_mul_fwd", mutates_args=())
 def gelu_mul_fwd(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     lib = _lib.load()
     av, M, lda = _as_rows(a)
@@ -866,7 +937,7 @@ def _(a, b):
     return a.new_empty(a.shape)
 
 
-@torch.library.custom_op("hawk_b200::gelu_mul_bwd", mutates_args=())
+@_operator("hawk_b200::gelu_mul_bwd", mutates_args=())
 def gelu_mul_bwd(dout: torch.Tensor, a: torch.Tensor, b: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     lib = _lib.load()
     J = a.shape[-1]
@@ -886,7 +957,7 @@ def _(dout, a, b):
     return a.new_empty(a.shape), a.new_empty(a.shape)
 
 
-@torch.library.custom_op("hawk_b200::gelu_mul_bwd_into", mutates_args=("da_out",))
+@_operator("hawk_b200::gelu_mul_bwd_into", mutates_args=("da_out",))
 def gelu_mul_bwd_into(dout: torch.Tensor, a: torch.Tensor, b: torch.Tensor, da_out: torch.Tensor) -> torch.Tensor:
     """gelu_mul_bwd with d a written into `da_out` (same shape as a; may be a row-strided view such as
     one half of a wider gradient buffer).  Returns d b."""
@@ -928,7 +999,7 @@ def gelu_mul(a, b):
     return gelu_mul_fwd(a, b)
 
 
-@torch.library.custom_op("hawk_b200::geglu_fwd", mutates_args=())
+@_operator("hawk_b200::geglu_fwd", mutates_args=())
 def geglu_fwd(gu: torch.Tensor) -> torch.Tensor:
     """gelu(gu[..., :I]) * gu[..., I:] for a contiguous [.., 2I] projection output."""
     lib = _lib.load()
@@ -948,7 +1019,7 @@ def _(gu):
     return gu.new_empty(*gu.shape[:-1], gu.shape[-1] // 2)
 
 
-@torch.library.custom_op("hawk_b200::geglu_bwd", mutates_args=())
+@_operator("hawk_b200::geglu_bwd", mutates_args=())
 def geglu_bwd(dout: torch.Tensor, gu: torch.Tensor) -> torch.Tensor:
     """Gradient of geglu_fwd w.r.t. gu: both halves written straight into one [.., 2I] buffer."""
     lib = _lib.load()
@@ -978,7 +1049,7 @@ def geglu(gu):
     return geglu_fwd(gu)
 
 
-@torch.library.custom_op("hawk_b200::rms_norm_fwd", mutates_args=())
+@_operator("hawk_b200::rms_norm_fwd", mutates_args=())
 def rms_norm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, out_dtype: torch.dtype) -> Tuple[torch.Tensor, torch.Tensor]:
     lib = _lib.load()
     x, w = x.contiguous(), w.contiguous()
@@ -997,7 +1068,7 @@ def _(x, w, eps, out_dtype):
     return x.new_empty(x.shape, dtype=out_dtype), x.new_empty(x.numel() // x.shape[-1], dtype=torch.float32)
 
 
-@torch.library.custom_op("hawk_b200::rms_norm_bwd", mutates_args=())
+@_operator("hawk_b200::rms_norm_bwd", mutates_args=())
 def rms_norm_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     lib = _lib.load()
     dy, x, w = dy.contiguous(), x.contiguous(), w.contiguous()
@@ -1122,7 +1193,7 @@ def gates_kernel_ok(x: torch.Tensor, nb: int, bw: int) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16 and R % 128 == 0 and 8 <= bw <= 128 and 128 % bw == 0
 
 
-@torch.library.custom_op("hawk_b200::gates_pack", mutates_args=())
+@_operator("hawk_b200::gates_pack", mutates_args=())
 def gates_pack(wx: torch.Tensor, wa: torch.Tensor) -> torch.Tensor:
     """Both gate weights [nb, bw, bw] (fp32 or bf16) in the operand layouts of gates_fwd / gates_bwd (bf16)."""
     lib = _lib.load()
@@ -1142,7 +1213,7 @@ def _(wx, wa):
     return wx.new_empty((nb * bw // 128) * (256 * 128 + 128 * 384), dtype=torch.bfloat16)
 
 
-@torch.library.custom_op("hawk_b200::gates_fwd", mutates_args=())
+@_operator("hawk_b200::gates_fwd", mutates_args=())
 def gates_fwd(xc: torch.Tensor, packed: torch.Tensor, bw: int) -> torch.Tensor:
     """[2, M, R]: (input-gate, recurrence-gate) projections of xc [M, R] bf16, without biases."""
     lib = _lib.load()
@@ -1160,7 +1231,7 @@ def _(xc, packed, bw):
     return xc.new_empty(2, xc.shape[0], xc.shape[1])
 
 
-@torch.library.custom_op("hawk_b200::gates_bwd_into", mutates_args=("dxc",))
+@_operator("hawk_b200::gates_bwd_into", mutates_args=("dxc",))
 def gates_bwd_into(xc: torch.Tensor, dgx: torch.Tensor, dga: torch.Tensor, packed: torch.Tensor, dxc: torch.Tensor,
                    bw: int) -> Tuple[torch.Tensor, torch.Tensor]:
     """dxc += dgx Wx^T + dga Wa^T in place (dxc [M, R] bf16 contiguous); returns (dwx, dwa) [nb, bw, bw] fp32."""
@@ -1189,7 +1260,7 @@ def _(xc, dgx, dga, packed, dxc, bw):
 # The strided-batch cuBLAS form of the same two projections for the cases the kernels do not take (fp32
 # activations, widths that are not multiples of 128), as opaque operators so that torch.compile traces
 # through the recurrent core without looking inside.
-@torch.library.custom_op("hawk_b200::gates_bmm_fwd", mutates_args=())
+@_operator("hawk_b200::gates_bmm_fwd", mutates_args=())
 def gates_bmm_fwd(xc: torch.Tensor, wx: torch.Tensor, wa: torch.Tensor) -> torch.Tensor:
     """[2, M, R] from xc [M, R] and weights [nb, bw, bw] already in xc's dtype; reads and writes the final
     layout in place (batch stride bw, row pitch R): no transposed copies."""
@@ -1207,7 +1278,7 @@ def _(xc, wx, wa):
     return xc.new_empty(2, xc.shape[0], xc.shape[1])
 
 
-@torch.library.custom_op("hawk_b200::gates_bmm_bwd_into", mutates_args=("dxc",))
+@_operator("hawk_b200::gates_bmm_bwd_into", mutates_args=("dxc",))
 def gates_bmm_bwd_into(xc: torch.Tensor, dgx: torch.Tensor, dga: torch.Tensor, wx: torch.Tensor, wa: torch.Tensor,
                        dxc: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """dxc += dgx Wx^T + dga Wa^T in place; returns (dwx, dwa) in the weights' dtype."""
@@ -1263,7 +1334,7 @@ def fused_block_diag_gates(x, wx, wa):
 # ---------------------------------------------------------------------------------------------
 # bf16 projection of an fp32 parameter (what autocast makes of nn.Linear), with fewer passes
 # ---------------------------------------------------------------------------------------------
-@torch.library.custom_op("hawk_b200::cast_bf16", mutates_args=())
+@_operator("hawk_b200::cast_bf16", mutates_args=())
 def cast_bf16(x: torch.Tensor) -> torch.Tensor:
     """fp32 -> bf16 copy of a contiguous tensor in one vectorised pass."""
     lib = _lib.load()
@@ -1392,7 +1463,7 @@ def recurrent_core(xy, conv_w, conv_b, wx, wa, gate_bias, lam):
 # ---------------------------------------------------------------------------------------------
 # residual add fused into the norm that follows it
 # ---------------------------------------------------------------------------------------------
-@torch.library.custom_op("hawk_b200::add_rms_norm_fwd", mutates_args=())
+@_operator("hawk_b200::add_rms_norm_fwd", mutates_args=())
 def add_rms_norm_fwd(res: torch.Tensor, delta: torch.Tensor, w: torch.Tensor, eps: float,
                      out_dtype: torch.dtype) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """(res + delta, rms_norm(res + delta) * w, rstd); delta must have dtype out_dtype."""
@@ -1416,7 +1487,7 @@ def _(res, delta, w, eps, out_dtype):
             res.new_empty(res.numel() // res.shape[-1], dtype=torch.float32))
 
 
-@torch.library.custom_op("hawk_b200::add_rms_norm_bwd", mutates_args=())
+@_operator("hawk_b200::add_rms_norm_bwd", mutates_args=())
 def add_rms_norm_bwd(gres: Optional[torch.Tensor], dy: torch.Tensor, x_sum: torch.Tensor, w: torch.Tensor,
                      rstd: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """(d res, d delta, d w): d res = gres + norm-backward(dy); d delta is the same in dy's dtype."""
