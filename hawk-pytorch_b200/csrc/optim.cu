@@ -1,4 +1,4 @@
-// AdamW update of one fp32 parameter tensor in a single pass, optionally emitting the bf16 copy of the
+// AdamW update of fp32 parameter tensors in a single pass, optionally emitting the bf16 copy of the
 // updated weights that the next step's bf16 GEMMs consume.  Training with torch.optim.AdamW under bf16
 // autocast makes an optimiser pass over p, g, m, v and then, at the next forward, a separate
 // fp32 -> bf16 cast pass per weight.  Here the cast rides on the update: 28 bytes per element read or
@@ -21,14 +21,37 @@ __device__ __forceinline__ float adamw_one(float p, float g, float& m, float& v,
   return p - a.step_size * (m / denom);
 }
 
-template <bool VEC4>
-__global__ void __launch_bounds__(256)
-adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-             __nv_bfloat16* __restrict__ p16, int64_t n, AdamwArgs a) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
-  if (VEC4) {
-    const int64_t nvec = n / 4;
-    for (int64_t i = tid; i < nvec; i += nthreads) {
+// One launch updates up to kAdamwTensors tensors: a model of 42 M parameters in 55 tensors spent 328 us in as many launches,
+// most of them a wave of a few blocks that start, read once and drain.  A block takes kAdamwChunk consecutive elements of
+// one tensor; the table with the tensors' addresses and first blocks comes as a kernel parameter (under 4 KB).
+constexpr int kAdamwTensors = 64, kAdamwChunk = 8192;
+
+struct AdamwTable {
+  hawk_adamw_tensor t[kAdamwTensors];
+  uint32_t first[kAdamwTensors + 1];  // first block of each tensor
+  uint8_t vec[kAdamwTensors];         // 16-byte accesses
+  int count;
+};
+
+__global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ AdamwTable tab, AdamwArgs a) {
+  int lo = 0, hi = tab.count;  // the tensor whose blocks hold this one
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (blockIdx.x >= tab.first[mid]) lo = mid; else hi = mid;
+  }
+  const hawk_adamw_tensor& t = tab.t[lo];
+  const int64_t i0 = (int64_t)(blockIdx.x - tab.first[lo]) * kAdamwChunk;
+  const int64_t n = t.n - i0 < kAdamwChunk ? t.n - i0 : kAdamwChunk;
+  float* p = t.p + i0;
+  const float* g = t.g + i0;
+  float* m = t.m + i0;
+  float* v = t.v + i0;
+  __nv_bfloat16* p16 = t.p_bf16 ? static_cast<__nv_bfloat16*>(t.p_bf16) + i0 : nullptr;
+  int64_t done = 0;
+  if (tab.vec[lo]) {
+    const int nvec = (int)(n / 4);
+#pragma unroll 2
+    for (int i = threadIdx.x; i < nvec; i += 256) {
       float4 pv = reinterpret_cast<float4*>(p)[i];
       const float4 gv = __ldg(reinterpret_cast<const float4*>(g) + i);
       float4 mv = reinterpret_cast<float4*>(m)[i], vv = reinterpret_cast<float4*>(v)[i];
@@ -42,19 +65,13 @@ adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restri
       if (p16 != nullptr)
         reinterpret_cast<uint2*>(p16)[i] = make_uint2(pack_bf16x2(pv.x, pv.y), pack_bf16x2(pv.z, pv.w));
     }
-    for (int64_t i = nvec * 4 + tid; i < n; i += nthreads) {  // ragged tail
-      float mm = m[i], vv = v[i];
-      const float pn = adamw_one(p[i], g[i], mm, vv, a);
-      p[i] = pn; m[i] = mm; v[i] = vv;
-      if (p16 != nullptr) p16[i] = __float2bfloat16(pn);
-    }
-  } else {
-    for (int64_t i = tid; i < n; i += nthreads) {
-      float mm = m[i], vv = v[i];
-      const float pn = adamw_one(p[i], g[i], mm, vv, a);
-      p[i] = pn; m[i] = mm; v[i] = vv;
-      if (p16 != nullptr) p16[i] = __float2bfloat16(pn);
-    }
+    done = (int64_t)nvec * 4;
+  }
+  for (int64_t i = done + threadIdx.x; i < n; i += 256) {  // ragged tail, or a tensor at an odd address
+    float mm = m[i], vv = v[i];
+    const float pn = adamw_one(p[i], g[i], mm, vv, a);
+    p[i] = pn; m[i] = mm; v[i] = vv;
+    if (p16 != nullptr) p16[i] = __float2bfloat16(pn);
   }
 }
 
@@ -62,11 +79,16 @@ adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restri
 
 using namespace hawk;
 
-extern "C" int hawk_adamw_step(float* p, const float* g, float* m, float* v, void* p_bf16, int64_t n, float lr,
-                               float beta1, float beta2, float eps, float weight_decay, int64_t step, void* stream) {
-  HAWK_REQUIRE(p && g && m && v, HAWK_ERR_NULL);
-  HAWK_REQUIRE(n >= 1 && step >= 1, HAWK_ERR_SHAPE);
-  HAWK_REQUIRE(aligned(p, 4) && aligned(g, 4) && aligned(m, 4) && aligned(v, 4) && aligned(p_bf16, 2), HAWK_ERR_ALIGN);
+extern "C" int hawk_adamw_multi(const hawk_adamw_tensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                                float weight_decay, int64_t step, void* stream) {
+  HAWK_REQUIRE(tensors, HAWK_ERR_NULL);
+  HAWK_REQUIRE(count >= 1 && step >= 1, HAWK_ERR_SHAPE);
+  for (int i = 0; i < count; ++i) {
+    const hawk_adamw_tensor& t = tensors[i];
+    HAWK_REQUIRE(t.p && t.g && t.m && t.v, HAWK_ERR_NULL);
+    HAWK_REQUIRE(t.n >= 1 && t.n <= (1LL << 40), HAWK_ERR_SHAPE);
+    HAWK_REQUIRE(aligned(t.p, 4) && aligned(t.g, 4) && aligned(t.m, 4) && aligned(t.v, 4) && aligned(t.p_bf16, 2), HAWK_ERR_ALIGN);
+  }
   AdamwArgs a;
   a.lr = lr;
   a.beta1 = beta1;
@@ -76,14 +98,31 @@ extern "C" int hawk_adamw_step(float* p, const float* g, float* m, float* v, voi
   const double bc1 = 1.0 - pow((double)beta1, (double)step), bc2 = 1.0 - pow((double)beta2, (double)step);
   a.step_size = (float)((double)lr / bc1);
   a.inv_sqrt_bc2 = (float)(1.0 / sqrt(bc2));
-  const bool vec = aligned(p, 16) && aligned(g, 16) && aligned(m, 16) && aligned(v, 16) && aligned(p_bf16, 8);
-  const int64_t work = vec ? (n + 3) / 4 : n;
-  const int64_t want = (work + 255) / 256, cap = 148LL * 8;
-  const unsigned grid = (unsigned)(want < cap ? want : cap);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (vec)
-    adamw_kernel<true><<<grid, 256, 0, st>>>(p, g, m, v, static_cast<__nv_bfloat16*>(p_bf16), n, a);
-  else
-    adamw_kernel<false><<<grid, 256, 0, st>>>(p, g, m, v, static_cast<__nv_bfloat16*>(p_bf16), n, a);
-  return launch_status();
+  for (int i0 = 0; i0 < count;) {
+    AdamwTable tab;
+    uint32_t blocks = 0;
+    int k = 0;
+    for (; k < kAdamwTensors && i0 + k < count; ++k) {
+      const hawk_adamw_tensor& t = tensors[i0 + k];
+      const int64_t need = (t.n + kAdamwChunk - 1) / kAdamwChunk;
+      if (need > (int64_t)0x7fffffff - blocks) break;  // the next launch's
+      tab.t[k] = t;
+      tab.first[k] = blocks;
+      tab.vec[k] = aligned(t.p, 16) && aligned(t.g, 16) && aligned(t.m, 16) && aligned(t.v, 16) && aligned(t.p_bf16, 8);
+      blocks += (uint32_t)need;
+    }
+    tab.first[k] = blocks;
+    tab.count = k;
+    adamw_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(tab, a);
+    const int rc = launch_status();
+    if (rc != HAWK_OK) return rc;
+    i0 += k;
+  }
+  return HAWK_OK;
+}
+
+extern "C" int hawk_adamw_step(float* p, const float* g, float* m, float* v, void* p_bf16, int64_t n, float lr,
+                               float beta1, float beta2, float eps, float weight_decay, int64_t step, void* stream) {
+  const hawk_adamw_tensor one = {p, g, m, v, p_bf16, n};
+  return hawk_adamw_multi(&one, 1, lr, beta1, beta2, eps, weight_decay, step, stream);
 }

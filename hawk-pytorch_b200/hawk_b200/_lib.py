@@ -55,6 +55,7 @@ SIGNATURES = {
     "hawk_decode_layer": (c_int, [ctypes.POINTER(DecodeLayerArgs), _P]),
     "hawk_decode_norm_linear": (c_int, [_P, _P, _P, c_float, _P, _P, _P, c_size_t] + [c_int] * 6 + [_P, _P]),
     "hawk_adamw_step": (c_int, [_P, _P, _P, _P, _P, c_int64, c_float, c_float, c_float, c_float, c_float, c_int64, _P]),
+    "hawk_adamw_multi": (c_int, [c_char_p, c_int, c_float, c_float, c_float, c_float, c_float, c_int64, _P]),
     "hawk_cast_f32_bf16": (c_int, [_P, _P, c_int64, _P]),
     "hawk_gelu_mul_fwd": (c_int, [_P, c_int64, _P, c_int64, _P, c_int64, c_int64, c_int, c_int, _P]),
     "hawk_gelu_mul_bwd": (c_int, [_P, c_int64, _P, c_int64, _P, c_int64, _P, c_int64, _P, c_int64, c_int64, c_int,

@@ -5,6 +5,7 @@ harness the multi-GPU benchmark and tests drive."""
 from __future__ import annotations
 
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -32,8 +33,8 @@ def init_distributed(backend: Optional[str] = None) -> tuple:
 
 
 class FusedAdamW(torch.optim.Optimizer):
-    """torch.optim.AdamW's update (decoupled weight decay, bias correction) with one kernel per fp32
-    parameter tensor that also writes the bf16 copy of the updated weight for the model's `Linear`
+    """torch.optim.AdamW's update (decoupled weight decay, bias correction) of fp32 parameters, up to 64 tensors
+    to a kernel that also writes the bf16 copy of the updated weight for the model's `Linear`
     layers (`shadow_modules`: modules with `.weight`, `.weight_bf16`, `.weight_bf16_version`), so the next
     forward casts nothing.  State keys follow torch.optim.AdamW (`step`, `exp_avg`, `exp_avg_sq`)."""
 
@@ -49,10 +50,11 @@ class FusedAdamW(torch.optim.Optimizer):
             with torch.enable_grad():
                 loss = closure()
         lib = _lib.load()
-        touched = []
+        touched, keep, launches = [], [], 0
         for group in self.param_groups:
             b1, b2 = group["betas"]
             lr, eps, wd = group["lr"], group["eps"], group["weight_decay"]
+            batches = {}  # (device, step) -> the addresses of its tensors, as hawk_adamw_tensor lays them out
             for p in group["params"]:
                 g = p.grad
                 if g is None:
@@ -63,21 +65,18 @@ class FusedAdamW(torch.optim.Optimizer):
                 st["step"] += 1
                 if not g.is_contiguous():
                     g = g.contiguous()
-                # pointers of p, m, v and the bf16 copy are fixed for the life of the state: one ctypes
-                # call per tensor with cached addresses keeps the host side of 300+ launches to ~2 ms
-                p_ptr, m_ptr, v_ptr, wb_ptr, n, dev = st["_args"]
-                if p_ptr != p.data_ptr():  # the parameter was moved or re-allocated since the state was made
+                    keep.append(g)
+                if st["_args"][0] != p.data_ptr():  # the parameter was moved or re-allocated since the state was made
                     self._bind(p, st)
-                    p_ptr, m_ptr, v_ptr, wb_ptr, n, dev = st["_args"]
-                if dev != torch.cuda.current_device():
-                    with torch.cuda.device(dev):
-                        rc = lib.hawk_adamw_step(p_ptr, g.data_ptr(), m_ptr, v_ptr, wb_ptr, n, lr, b1, b2, eps, wd,
-                                                 st["step"], torch.cuda.current_stream().cuda_stream)
-                else:
-                    rc = lib.hawk_adamw_step(p_ptr, g.data_ptr(), m_ptr, v_ptr, wb_ptr, n, lr, b1, b2, eps, wd,
-                                             st["step"], torch.cuda.current_stream().cuda_stream)
-                _lib.check(rc, "hawk_adamw_step")
+                p_ptr, m_ptr, v_ptr, wb_ptr, n, dev = st["_args"]
+                batches.setdefault((dev, st["step"]), []).extend((p_ptr, g.data_ptr(), m_ptr, v_ptr, wb_ptr or 0, n))
                 touched.append(p)
+            for (dev, step), flat in batches.items():
+                with torch.cuda.device(dev):
+                    rc = lib.hawk_adamw_multi(struct.pack(f"{len(flat)}Q", *flat), len(flat) // 6, lr, b1, b2, eps, wd, step,
+                                              torch.cuda.current_stream().cuda_stream)
+                _lib.check(rc, "hawk_adamw_multi")
+                launches += (len(flat) // 6 + 63) // 64
         if touched:
             torch.autograd.graph.increment_version(touched)  # the kernels wrote p behind autograd's back
             for p in touched:
@@ -85,7 +84,7 @@ class FusedAdamW(torch.optim.Optimizer):
                 if mod is not None:
                     mod.weight_bf16, mod.weight_bf16_version = self.state[p]["_shadow"], p._version
             if ops.LOG.enabled:
-                ops.LOG.counts["adamw_step"] = ops.LOG.counts.get("adamw_step", 0) + len(touched)
+                ops.LOG.counts["adamw_step"] = ops.LOG.counts.get("adamw_step", 0) + launches
         return loss
 
     def _init_state(self, p, st):

@@ -345,6 +345,16 @@ int hawk_cast_f32_bf16(const float* src, void* dst, int64_t n, void* stream);
  * (README.md:36) and leaves the optimiser to the user; this is the update torch.optim.AdamW would make. */
 int hawk_adamw_step(float* p, const float* g, float* m, float* v, void* p_bf16, int64_t n, float lr, float beta1,
                     float beta2, float eps, float weight_decay, int64_t step, void* stream);
+/* The same for `count` tensors (a host array) in one launch per 64 of them. */
+typedef struct hawk_adamw_tensor {
+  float* p;
+  const float* g;
+  float *m, *v;
+  void* p_bf16; /* NULL: no bf16 copy */
+  int64_t n;
+} hawk_adamw_tensor;
+int hawk_adamw_multi(const hawk_adamw_tensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                     float weight_decay, int64_t step, void* stream);
 
 #ifdef __cplusplus
 }

@@ -87,3 +87,24 @@ def test_trainer_keeps_bf16_weight_copies_current():
     assert m.weight_bf16 is None
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert torch.equal(m(x), torch.nn.functional.linear(x, m.weight))  # ... not after dropping it
+
+
+def test_fused_adamw_many_tensors_around_its_chunks():
+    """More tensors than one launch takes, at sizes around a block's 8192 elements, some at addresses that rule out 16-byte
+    accesses; a second group and a parameter that skips a step (another bias correction) among them."""
+    from hawk_b200.train import FusedAdamW
+    sizes = [1, 3, 8191, 8192, 8193, 16384, 16389] * 11
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mine = [torch.nn.Parameter(torch.randn(n + 1, generator=g, device="cuda")[i % 2:n + i % 2]) for i, n in enumerate(sizes)]
+    ref = [torch.nn.Parameter(p.detach().clone()) for p in mine]
+    groups = lambda ps: [dict(params=ps[:70]), dict(params=ps[70:], lr=1e-2, weight_decay=0.0)]
+    kw = dict(lr=3e-3, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1)
+    o1, o2 = FusedAdamW(groups(mine), **kw), torch.optim.AdamW(groups(ref), foreach=False, fused=False, **kw)
+    for step in range(3):
+        for i, (a, b) in enumerate(zip(mine, ref)):
+            gr = torch.randn(a.shape, generator=g, device="cuda")
+            a.grad, b.grad = (None, None) if (i == 5 and step == 1) else (gr.clone(), gr.clone())
+        o1.step()
+        o2.step()
+    for a, b in zip(mine, ref):  # the bound of the test above
+        assert float((a - b).abs().max()) <= 2e-6 * float(b.abs().max())
