@@ -129,6 +129,38 @@ __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restr
   }
 }
 
+// ---- small launches of a block's forward without gradients, folded into one each ------------------------------------
+// out = the fp32 values of conv_w [W,R], conv_b, bx, ba, lam [R each], one after the other.  As torch operations: a cast of
+// each and a stack of the gate biases, six launches per layer of a bf16 model.
+struct CoreParams {
+  const void* src[5];
+  int bf16[5];
+};
+__global__ void __launch_bounds__(256) core_params_kernel(CoreParams p, float* __restrict__ out, int W, int R) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= (W + 4) * R) return;
+  const int seg = i < W * R ? 0 : 1 + (i - W * R) / R;
+  const int o = seg == 0 ? i : i - (W + seg - 1) * R;
+  out[i] = p.bf16[seg] ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.src[seg])[o]) : static_cast<const float*>(p.src[seg])[o];
+}
+
+// The decode state that a prompt leaves behind: conv_state [B,keep,R] = the last `keep` rows of x (zero before its first),
+// state [B,R] = the last row of h [B,T,R].
+template <typename T, typename TS>
+__global__ void __launch_bounds__(256)
+cache_store_kernel(const T* __restrict__ x, int64_t bs, int64_t ld, const T* __restrict__ h, TS* __restrict__ conv_state,
+                   TS* __restrict__ state, int B, int T_len, int R, int keep) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (int64_t)B * (keep + 1) * R) return;
+  const int c = (int)(i % R), j = (int)(i / R % (keep + 1)), b = (int)(i / R / (keep + 1));
+  if (j == keep) {
+    state[(int64_t)b * R + c] = from_float<TS>(to_float(h[((int64_t)b * T_len + T_len - 1) * R + c]));
+  } else {
+    const int t = T_len - keep + j;
+    conv_state[((int64_t)b * keep + j) * R + c] = from_float<TS>(t >= 0 ? to_float(x[b * bs + t * ld + c]) : 0.f);
+  }
+}
+
 // ---- RMSNorm: one warp per row, two passes over the row (the second hits L1/L2) ----------------
 // With `delta` the row is first updated, x_out = x + delta (the residual add that precedes every norm
 // in the block, hawk/hawk.py:229-234), and the norm is taken of the sum: one pass instead of two ops.
@@ -466,6 +498,39 @@ extern "C" int hawk_cast_f32_bf16(const float* src, void* dst, int64_t n, void* 
   HAWK_REQUIRE(aligned(src, 16) && aligned(dst, 16), HAWK_ERR_ALIGN);
   cast_f32_bf16_kernel<<<grid_for(n / 8 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       src, static_cast<bf*>(dst), n);
+  return launch_status();
+}
+
+extern "C" int hawk_core_params(const void* conv_w, int conv_w_dtype, const void* conv_b, int conv_b_dtype, const void* bx,
+                                int bx_dtype, const void* ba, int ba_dtype, const void* lam, int lam_dtype, float* out, int W,
+                                int R, void* stream) {
+  HAWK_REQUIRE(conv_w && conv_b && bx && ba && lam && out, HAWK_ERR_NULL);
+  const CoreParams p = {{conv_w, conv_b, bx, ba, lam},
+                        {conv_w_dtype == HAWK_BF16, conv_b_dtype == HAWK_BF16, bx_dtype == HAWK_BF16, ba_dtype == HAWK_BF16,
+                         lam_dtype == HAWK_BF16}};
+  HAWK_REQUIRE(valid_dtype(conv_w_dtype) && valid_dtype(conv_b_dtype) && valid_dtype(bx_dtype) && valid_dtype(ba_dtype) &&
+                   valid_dtype(lam_dtype),
+               HAWK_ERR_DTYPE);
+  HAWK_REQUIRE(W >= 1 && W <= 64 && R >= 1 && R <= (1 << 24), HAWK_ERR_SHAPE);
+  core_params_kernel<<<(unsigned)(((W + 4) * R + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, out, W, R);
+  return launch_status();
+}
+
+extern "C" int hawk_cache_store(const void* x, int64_t x_batch_stride, int64_t x_row_stride, const void* h, void* conv_state,
+                                void* state, int B, int T, int R, int keep, int dtype, int state_dtype, void* stream) {
+  HAWK_REQUIRE(x && h && state && (conv_state || keep == 0), HAWK_ERR_NULL);
+  HAWK_REQUIRE(valid_dtype(dtype) && valid_dtype(state_dtype), HAWK_ERR_DTYPE);
+  HAWK_REQUIRE(B >= 1 && T >= 1 && R >= 1 && keep >= 0 && (int64_t)B * (keep + 1) * R <= (1LL << 38), HAWK_ERR_SHAPE);
+  const unsigned blocks = (unsigned)(((int64_t)B * (keep + 1) * R + 255) / 256);
+  auto go = [&](auto tx, auto ts) {
+    using T_ = decltype(tx);
+    using TS = decltype(ts);
+    cache_store_kernel<T_, TS><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const T_*>(x), x_batch_stride, x_row_stride, static_cast<const T_*>(h), static_cast<TS*>(conv_state),
+        static_cast<TS*>(state), B, T, R, keep);
+  };
+  if (dtype == HAWK_BF16) state_dtype == HAWK_BF16 ? go(bf{}, bf{}) : go(bf{}, 0.f);
+  else state_dtype == HAWK_BF16 ? go(0.f, bf{}) : go(0.f, 0.f);
   return launch_status();
 }
 

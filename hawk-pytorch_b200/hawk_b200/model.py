@@ -264,15 +264,31 @@ class Hawk(nn.Module):
         # conv -> gates -> scan -> gelu(y) * h as one autograd node; the gate biases go to the scan kernel,
         # which adds them for free and sums their gradients
         conv = self.conv1d
-        gate_bias = torch.stack((self.rg_lru_input_gate.b.reshape(-1), self.rg_lru_a_gate.b.reshape(-1))).float()
-        out, h = ops.recurrent_core(xb_y, self._fp32("w", conv.w) if not conv.w.requires_grad else conv.w.float(),
-                                    self._fp32("b", conv.b) if not conv.b.requires_grad else conv.b.float(),
-                                    self.rg_lru_input_gate.w, self.rg_lru_a_gate.w, gate_bias,
-                                    self.rg_lru_a_param.float())
+        gi, ga_ = self.rg_lru_input_gate, self.rg_lru_a_gate
+        small = (conv.w, conv.b, gi.b, ga_.b, self.rg_lru_a_param)
+        if (not torch.is_grad_enabled() and x.is_cuda and any(p.dtype == torch.bfloat16 for p in small)
+                and all(p.dtype in (torch.float32, torch.bfloat16) for p in small)):
+            W, R = conv.w.shape  # a reduced-precision model: all five in fp32 by one launch
+            buf = ops.core_params(*small)
+            cw, cb, gate_bias, lam = buf[:W * R].view(W, R), buf[W * R:][:R], buf[(W + 1) * R:][:2 * R].view(2, R), buf[-R:]
+        else:
+            gate_bias = torch.stack((gi.b.reshape(-1), ga_.b.reshape(-1))).float()
+            cw = self._fp32("w", conv.w) if not conv.w.requires_grad else conv.w.float()
+            cb = self._fp32("b", conv.b) if not conv.b.requires_grad else conv.b.float()
+            lam = self.rg_lru_a_param.float()
+        out, h = ops.recurrent_core(xb_y, cw, cb, gi.w, ga_.w, gate_bias, lam)
         cache = None
         if self.use_cache:
             assert layer_past is not None, "use_cache=True needs an RNNCache per layer"
             keep = layer_past.conv_cache_size
+            states = (layer_past.conv_state, layer_past.recc_state)
+            if (type(layer_past) is RNNCache and not torch.is_grad_enabled() and x.is_cuda and h.dtype == xb.dtype
+                    and states[0].shape == (xb.shape[0], keep, xb.shape[2]) and states[1].shape == h[:, -1:].shape
+                    and states[0].dtype == states[1].dtype and states[0].dtype in (torch.float32, torch.bfloat16)
+                    and all(t.is_contiguous() and t.device == x.device for t in states)):
+                ops.cache_store(xb, h, *states)
+                layer_past.current_cache_size = 1
+                return self.resid_proj(out), layer_past
             tail = xb[:, -keep:]
             if tail.shape[1] < keep:  # prompt shorter than the conv history: zero history before it
                 tail = F.pad(tail, (0, 0, keep - tail.shape[1], 0))

@@ -665,6 +665,48 @@ def _(x, gx, ga, lam, state):
     return torch.empty_like(x)
 
 
+@_operator("hawk_b200::core_params", mutates_args=())
+def core_params(conv_w: torch.Tensor, conv_b: torch.Tensor, bx: torch.Tensor, ba: torch.Tensor, lam: torch.Tensor) -> torch.Tensor:
+    """fp32 values of conv_w [W,R], conv_b [R], the gate biases [nb,bw] and Lambda [R], one after the other."""
+    lib = _lib.load()
+    W, R = conv_w.shape
+    assert conv_b.numel() == bx.numel() == ba.numel() == lam.numel() == R
+    conv_w, conv_b, bx, ba, lam = (t.contiguous() for t in (conv_w, conv_b, bx, ba, lam))
+    out = torch.empty((W + 4) * R, dtype=torch.float32, device=conv_w.device)
+    with _on(conv_w, "core_params", 1):
+        _lib.check(lib.hawk_core_params(conv_w.data_ptr(), _dt(conv_w), conv_b.data_ptr(), _dt(conv_b), bx.data_ptr(), _dt(bx),
+                                        ba.data_ptr(), _dt(ba), lam.data_ptr(), _dt(lam), out.data_ptr(), W, R,
+                                        _stream(conv_w)), "hawk_core_params")
+    return out
+
+
+@core_params.register_fake
+def _(conv_w, conv_b, bx, ba, lam):
+    return conv_w.new_empty(conv_w.numel() + 4 * conv_w.shape[1], dtype=torch.float32)
+
+
+@_operator("hawk_b200::cache_store", mutates_args=("conv_state", "state"))
+def cache_store(x: torch.Tensor, h: torch.Tensor, conv_state: torch.Tensor, state: torch.Tensor) -> None:
+    """The decode caches after a prompt: conv_state [B,keep,R] takes the last rows of x [B,T,R] (zero before its first one;
+    x may be row-strided), state [B,1,R] the last row of h [B,T,R]."""
+    lib = _lib.load()
+    B, T, R = x.shape
+    keep = conv_state.shape[1]
+    assert h.shape == x.shape and h.dtype == x.dtype and conv_state.shape == (B, keep, R) and state.numel() == B * R
+    assert conv_state.is_contiguous() and state.is_contiguous() and conv_state.dtype == state.dtype
+    if x.stride(2) != 1:
+        x = x.contiguous()
+    h = h.contiguous()
+    with _on(x, "cache_store", 1):
+        _lib.check(lib.hawk_cache_store(x.data_ptr(), x.stride(0), x.stride(1), h.data_ptr(), conv_state.data_ptr(),
+                                        state.data_ptr(), B, T, R, keep, _dt(x), _dt(state), _stream(x)), "hawk_cache_store")
+
+
+@cache_store.register_fake
+def _(x, h, conv_state, state):
+    return None
+
+
 def _dense16(t: torch.Tensor) -> torch.Tensor:
     """t contiguous at a 16-byte aligned address."""
     t = t.contiguous()

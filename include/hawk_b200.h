@@ -223,6 +223,15 @@ int hawk_decode_norm_linear(const void* residual, const void* pending, const flo
                             void* workspace, size_t workspace_bytes, int B, int H, int N, int res_dtype, int w_dtype,
                             int follows_layer, int* status, void* stream);
 
+/* The block's forward without gradients, between its large kernels: the fp32 values of conv_w [W,R], conv_b, bx, ba, lam [R]
+ * one after the other in out [(W + 4) * R]; and the caches after a prompt: conv_state [B,keep,R] = the last keep rows of the
+ * conv's input x [B,T,R] (strides in elements; zero before its first row, hawk/hawk.py:184-190), state [B,R] = the last row of
+ * h [B,T,R]. */
+int hawk_core_params(const void* conv_w, int conv_w_dtype, const void* conv_b, int conv_b_dtype, const void* bx, int bx_dtype,
+                     const void* ba, int ba_dtype, const void* lam, int lam_dtype, float* out, int W, int R, void* stream);
+int hawk_cache_store(const void* x, int64_t x_batch_stride, int64_t x_row_stride, const void* h, void* conv_state, void* state,
+                     int B, int T, int R, int keep, int dtype, int state_dtype, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Fused linear + cross-entropy.  Replaces CrossEntropyLoopedFused.forward
  * (hawk/fused_cross_entropy.py:13-64): mean cross-entropy of act @ weight^T against labels, and

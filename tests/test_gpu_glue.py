@@ -239,3 +239,19 @@ def test_autocast_linear_matches_f_linear(lead, K, N):
     xd, wd = x.cuda().requires_grad_(True), w.cuda().requires_grad_(True)
     y = ops.linear(xd, wd)  # no autocast: plain fp32 F.linear
     assert y.dtype == torch.float32 and rel_l2(y.detach().cpu(), F.linear(x, w)) <= 2e-3
+
+
+@pytest.mark.parametrize("W,R,T", [(4, 64, 1), (4, 192, 2), (4, 512, 3), (2, 64, 9), (1, 64, 5)])
+@pytest.mark.parametrize("cache_dtype", [torch.bfloat16, torch.float32])
+def test_core_params_and_cache_store(W, R, T, cache_dtype):
+    from hawk_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(W + R + T)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ps = [r(W, R).bfloat16(), r(R), r(R // 16, 16).bfloat16(), r(R // 16, 16), r(R).bfloat16()]
+    assert torch.equal(ops.core_params(*ps), torch.cat([p.float().reshape(-1) for p in ps]))
+    x, h = r(3, T, 2 * R).bfloat16()[..., R:], r(3, T, R).bfloat16()
+    conv, state = torch.full((3, W - 1, R), 7.0, device="cuda").to(cache_dtype), r(3, 1, R).to(cache_dtype)
+    v = state._version
+    ops.cache_store(x, h, conv, state)
+    want = torch.cat([torch.zeros(3, W - 1, R, device="cuda"), x.float()], 1)[:, T:].to(cache_dtype)
+    assert torch.equal(conv, want) and torch.equal(state, h[:, -1:].to(cache_dtype)) and state._version > v
