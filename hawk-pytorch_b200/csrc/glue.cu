@@ -5,6 +5,8 @@
 // strided chunk views (non-vectorised).  Here every tensor is read once and written once with 16-byte
 // accesses; a and b may be row-strided views (the halves of a projection output), and the backward of
 // gelu_mul can write both gradients into the two halves of one buffer, so no concatenation is needed.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace hawk {
@@ -236,22 +238,39 @@ rms_norm_fwd_kernel(const TX* __restrict__ x, const TY* __restrict__ delta, TX* 
   }
 }
 
-// The same forward for H = 512 * NCH (NCH = 1, 2, 4, 8): one row per 128-thread group, kept in
-// registers between the sum of squares and the scaling, so the row is read once (see the backward
-// below for the group barrier).
-template <typename TX, typename TY, int NCH>
+// Sum of v over the TPR threads of a row's group.  A group of one warp needs no barrier; larger ones meet once at a named
+// barrier, with `part` double-buffered by the caller so that one per row is enough.
+template <int TPR>
+__device__ __forceinline__ float row_sum(float v, float (&part)[TPR / 32], int grp, int lane, int wig) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (TPR == 32) return v;
+  if (lane == 0) part[wig] = v;
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(TPR) : "memory");
+  v = part[0];
+#pragma unroll
+  for (int k = 1; k < TPR / 32; ++k) v += part[k];
+  return v;
+}
+
+// The same forward for H = 4 * TPR * NCH: one row per TPR threads, kept in registers between the sum of squares and the
+// scaling, so the row is read once.  What bounds it is bytes in flight: a thread's loads of one row are all it has
+// outstanding.  With 128 threads to a row of 512 that was one 16-byte load per tensor (N32768, fp32 stream, bf16 branch:
+// 42.2 us forward, 60.3 us backward, 4.8 and 4.4 TB/s); a warp to a row has four of each.  Groups are the narrowest that
+// keep a row's state in registers (NCH = 4), 128 threads from H = 1536 on.
+template <typename TX, typename TY, int TPR, int NCH>
 __global__ void __launch_bounds__(256, (NCH >= 8 ? 2 : 3))
 rms_norm_fwd_rows_kernel(const TX* __restrict__ x, const TY* __restrict__ delta, TX* __restrict__ x_out,
                          const float* __restrict__ w, TY* __restrict__ y, float* __restrict__ rstd, int64_t M,
                          float eps) {
-  constexpr int VEC = 4, TPR = 128, H = NCH * TPR * VEC;
-  __shared__ float part[2][2][4];
-  const int grp = threadIdx.x >> 7, t = threadIdx.x & (TPR - 1), lane = threadIdx.x & 31, wig = t >> 5;
+  constexpr int VEC = 4, H = NCH * TPR * VEC, GROUPS = 256 / TPR;
+  __shared__ float part[GROUPS][2][TPR / 32];
+  const int grp = threadIdx.x / TPR, t = threadIdx.x & (TPR - 1), lane = threadIdx.x & 31, wig = t >> 5;
   float wv[NCH][VEC];
 #pragma unroll
   for (int c = 0; c < NCH; ++c) VecIO<float, VEC>::load(w + (c * TPR + t) * VEC, wv[c]);
   int par = 0;
-  for (int64_t m = (int64_t)blockIdx.x * 2 + grp; m < M; m += (int64_t)gridDim.x * 2) {
+  for (int64_t m = (int64_t)blockIdx.x * GROUPS + grp; m < M; m += (int64_t)gridDim.x * GROUPS) {
     const int64_t row = m * H;
     float v[NCH][VEC];
 #pragma unroll
@@ -276,11 +295,7 @@ rms_norm_fwd_rows_kernel(const TX* __restrict__ x, const TY* __restrict__ delta,
     for (int c = 0; c < NCH; ++c)
 #pragma unroll
       for (int q = 0; q < VEC; ++q) ss = fmaf(v[c][q], v[c][q], ss);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) part[grp][par][wig] = ss;
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(TPR) : "memory");
-    ss = ((part[grp][par][0] + part[grp][par][1]) + part[grp][par][2]) + part[grp][par][3];
+    ss = row_sum<TPR>(ss, part[grp][par], grp, lane, wig);
     par ^= 1;
     const float inv = rsqrtf(ss / (float)H + eps);
     if (t == 0) rstd[m] = inv;
@@ -376,22 +391,19 @@ rms_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, const f
   }
 }
 
-// The same backward for H = 512 * NCH (NCH = 1, 2, 4, 8), one row per 128 threads, the row held in
-// registers between the dot product and the update: every input byte is loaded exactly once, all of a
-// row's loads (x, dy and the residual gradient: 10 x 16 bytes per thread at H = 2048) are in flight
-// together, and w is loaded once per thread because a thread keeps its columns for every row.  A CTA is two
-// independent row groups; a group's four warps meet once per row at a named barrier to sum the dot
-// product (double-buffered partials, so one barrier per row suffices).  dw partials: per-thread
-// column sums, the two groups added in shared memory, one partial row per CTA.
-template <typename TX, typename TY, int NCH>
+// The same backward for H = 4 * TPR * NCH, one row per TPR threads, the row held in registers between the dot product and
+// the update: every input byte is loaded exactly once, all of a row's loads (x, dy and the residual gradient: 12 x 16 bytes
+// per thread at NCH = 4) are in flight together, and w is loaded once per thread because a thread keeps its columns for
+// every row.  dw partials: per-thread column sums, the CTA's groups added in shared memory, one partial row per CTA.
+template <typename TX, typename TY, int TPR, int NCH>
 __global__ void __launch_bounds__(256, (NCH >= 8 ? 1 : 2))
 rms_norm_bwd_rows_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, const float* __restrict__ w,
                          const float* __restrict__ rstd, const TX* __restrict__ gres, TX* __restrict__ dx,
                          TY* __restrict__ ddelta, float* __restrict__ dw_partial, int64_t M) {
-  constexpr int VEC = 4, TPR = 128, H = NCH * TPR * VEC;
-  __shared__ float part[2][2][4];         // [group][parity][warp of the group]
-  __shared__ float other[TPR * NCH * VEC];  // group 1's column sums
-  const int grp = threadIdx.x >> 7, t = threadIdx.x & (TPR - 1), lane = threadIdx.x & 31, wig = t >> 5;
+  constexpr int VEC = 4, H = NCH * TPR * VEC, GROUPS = 256 / TPR;
+  __shared__ float part[GROUPS][2][TPR / 32];          // [group][parity][warp of the group]
+  __shared__ __align__(16) float other[GROUPS - 1][H];  // column sums of the groups but the first
+  const int grp = threadIdx.x / TPR, t = threadIdx.x & (TPR - 1), lane = threadIdx.x & 31, wig = t >> 5;
   float wv[NCH][VEC], acc[NCH][VEC];
 #pragma unroll
   for (int c = 0; c < NCH; ++c) {
@@ -400,7 +412,7 @@ rms_norm_bwd_rows_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, co
     for (int q = 0; q < VEC; ++q) acc[c][q] = 0.f;
   }
   int par = 0;
-  for (int64_t m = (int64_t)blockIdx.x * 2 + grp; m < M; m += (int64_t)gridDim.x * 2) {
+  for (int64_t m = (int64_t)blockIdx.x * GROUPS + grp; m < M; m += (int64_t)gridDim.x * GROUPS) {
     const int64_t row = m * H;
     float xv[NCH][VEC], gv[NCH][VEC], rv[NCH][VEC];
 #pragma unroll
@@ -422,11 +434,7 @@ rms_norm_bwd_rows_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, co
         gv[c][q] *= wv[c][q];                             // g = dy * w
         dot = fmaf(gv[c][q], xv[c][q], dot);
       }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if (lane == 0) part[grp][par][wig] = dot;
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(TPR) : "memory");
-    const float cmean = (((part[grp][par][0] + part[grp][par][1]) + part[grp][par][2]) + part[grp][par][3]) / (float)H;
+    const float cmean = row_sum<TPR>(dot, part[grp][par], grp, lane, wig) / (float)H;
     par ^= 1;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
@@ -440,11 +448,11 @@ rms_norm_bwd_rows_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, co
       if (ddelta != nullptr) VecIO<TY, VEC>::store(ddelta + row + (c * TPR + t) * VEC, o);  // same value, delta's dtype
     }
   }
-  if (grp == 1) {
+  if (grp > 0) {
 #pragma unroll
     for (int c = 0; c < NCH; ++c)
 #pragma unroll
-      for (int q = 0; q < VEC; ++q) other[(c * TPR + t) * VEC + q] = acc[c][q];
+      for (int q = 0; q < VEC; ++q) other[grp - 1][(c * TPR + t) * VEC + q] = acc[c][q];
   }
   __syncthreads();
   if (grp == 0) {
@@ -452,7 +460,10 @@ rms_norm_bwd_rows_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, co
     for (int c = 0; c < NCH; ++c) {
       float o[VEC];
 #pragma unroll
-      for (int q = 0; q < VEC; ++q) o[q] = acc[c][q] + other[(c * TPR + t) * VEC + q];
+      for (int q = 0; q < VEC; ++q) {
+        o[q] = acc[c][q];
+        for (int k = 0; k < GROUPS - 1; ++k) o[q] += other[k][(c * TPR + t) * VEC + q];
+      }
       VecIO<float, VEC>::store(dw_partial + (int64_t)blockIdx.x * H + (c * TPR + t) * VEC, o);
     }
   }
@@ -467,6 +478,7 @@ __global__ void __launch_bounds__(256) rows_sum_kernel(const float* __restrict__
   const int j = blockIdx.x * 32 + tx;
   float s = 0.f;
   if (j < H)
+#pragma unroll 8  // eight loads in flight; the order of the sum is the loop's
     for (int r = ty; r < rows; r += 8) s += partial[(int64_t)r * H + j];
   sl[ty][tx] = s;
   __syncthreads();
@@ -579,6 +591,23 @@ extern "C" int hawk_gelu_mul_bwd(const void* dout, int64_t ldd, const void* a, i
   return launch_status();
 }
 
+// widths of the rows-in-registers kernels; any other H takes the warp-per-row kernels, which read a row twice
+static bool norm_rows_width(int H) {
+  return H == 256 || H == 512 || H == 768 || H == 1024 || H == 1536 || H == 2048 || H == 4096;
+}
+#define HAWK_NORM_WIDTHS(LAUNCH, TX, TY)          \
+  do {                                            \
+    switch (H) {                                  \
+      case 256: LAUNCH(TX, TY, 32, 2); break;     \
+      case 512: LAUNCH(TX, TY, 32, 4); break;     \
+      case 768: LAUNCH(TX, TY, 64, 3); break;     \
+      case 1024: LAUNCH(TX, TY, 64, 4); break;    \
+      case 1536: LAUNCH(TX, TY, 128, 3); break;   \
+      case 2048: LAUNCH(TX, TY, 128, 4); break;   \
+      default: LAUNCH(TX, TY, 128, 8); break;     \
+    }                                             \
+  } while (0)
+
 static int norm_fwd_impl(const void* x, const void* delta, void* x_out, const float* w, void* y, float* rstd,
                          int64_t M, int H, float eps, int x_dtype, int y_dtype, cudaStream_t st) {
   HAWK_REQUIRE(x && w && y && rstd && ((delta == nullptr) == (x_out == nullptr)), HAWK_ERR_NULL);
@@ -586,18 +615,11 @@ static int norm_fwd_impl(const void* x, const void* delta, void* x_out, const fl
   HAWK_REQUIRE(M >= 1 && H >= 4 && H % 4 == 0, HAWK_ERR_SHAPE);
   HAWK_REQUIRE(aligned(x, 16) && aligned(w, 16) && aligned(y, 16) && aligned(delta, 16) && aligned(x_out, 16),
                HAWK_ERR_ALIGN);
-  if (H == 512 || H == 1024 || H == 2048 || H == 4096) {  // rows-in-registers path
-    const unsigned rgrid = (unsigned)(M / 2 + 1 < 148 * 3 ? M / 2 + 1 : 148 * 3);
-#define HAWK_NORM_FROWS_N(TX, TY, N)                                                                               \
-  rms_norm_fwd_rows_kernel<TX, TY, N><<<rgrid, 256, 0, st>>>(static_cast<const TX*>(x), static_cast<const TY*>(delta), \
-                                                             static_cast<TX*>(x_out), w, static_cast<TY*>(y), rstd, M, eps)
-#define HAWK_NORM_FROWS(TX, TY)                        \
-  do {                                                 \
-    if (H == 512) HAWK_NORM_FROWS_N(TX, TY, 1);        \
-    else if (H == 1024) HAWK_NORM_FROWS_N(TX, TY, 2);  \
-    else if (H == 2048) HAWK_NORM_FROWS_N(TX, TY, 4);  \
-    else HAWK_NORM_FROWS_N(TX, TY, 8);                 \
-  } while (0)
+  if (norm_rows_width(H)) {  // rows-in-registers path
+#define HAWK_NORM_FROWS_N(TX, TY, TPR, N)                                                                                  \
+  rms_norm_fwd_rows_kernel<TX, TY, TPR, N><<<(unsigned)std::min<int64_t>((M + 256 / TPR - 1) / (256 / TPR), 148 * 3), 256, 0, st>>>( \
+      static_cast<const TX*>(x), static_cast<const TY*>(delta), static_cast<TX*>(x_out), w, static_cast<TY*>(y), rstd, M, eps)
+#define HAWK_NORM_FROWS(TX, TY) HAWK_NORM_WIDTHS(HAWK_NORM_FROWS_N, TX, TY)
     if (x_dtype == HAWK_F32 && y_dtype == HAWK_BF16) HAWK_NORM_FROWS(float, bf);
     else if (x_dtype == HAWK_F32) HAWK_NORM_FROWS(float, float);
     else if (y_dtype == HAWK_BF16) HAWK_NORM_FROWS(bf, bf);
@@ -645,18 +667,12 @@ static int norm_bwd_impl(const void* dy, const void* x, const float* w, const fl
                    aligned(gres, 16) && aligned(ddelta, 16),
                HAWK_ERR_ALIGN);
   float* partial = static_cast<float*>(workspace);
-  if (H % 512 == 0 && (H == 512 || H == 1024 || H == 2048 || H == 4096)) {  // rows-in-registers path
-#define HAWK_NORM_ROWS_N(TX, TY, N)                                                                                   \
-  rms_norm_bwd_rows_kernel<TX, TY, N><<<kNormBwdCtas, 256, 0, st>>>(                                                  \
+  if (norm_rows_width(H)) {  // rows-in-registers path
+#define HAWK_NORM_ROWS_N(TX, TY, TPR, N)                                                                              \
+  rms_norm_bwd_rows_kernel<TX, TY, TPR, N><<<kNormBwdCtas, 256, 0, st>>>(                                                  \
       static_cast<const TY*>(dy), static_cast<const TX*>(x), w, rstd, static_cast<const TX*>(gres),                   \
       static_cast<TX*>(dx), static_cast<TY*>(ddelta), partial, M)
-#define HAWK_NORM_ROWS(TX, TY)                        \
-  do {                                                \
-    if (H == 512) HAWK_NORM_ROWS_N(TX, TY, 1);        \
-    else if (H == 1024) HAWK_NORM_ROWS_N(TX, TY, 2);  \
-    else if (H == 2048) HAWK_NORM_ROWS_N(TX, TY, 4);  \
-    else HAWK_NORM_ROWS_N(TX, TY, 8);                 \
-  } while (0)
+#define HAWK_NORM_ROWS(TX, TY) HAWK_NORM_WIDTHS(HAWK_NORM_ROWS_N, TX, TY)
     if (x_dtype == HAWK_F32 && y_dtype == HAWK_BF16) HAWK_NORM_ROWS(float, bf);
     else if (x_dtype == HAWK_F32) HAWK_NORM_ROWS(float, float);
     else if (y_dtype == HAWK_BF16) HAWK_NORM_ROWS(bf, bf);

@@ -241,6 +241,13 @@ def test_autocast_linear_matches_f_linear(lead, K, N):
     assert y.dtype == torch.float32 and rel_l2(y.detach().cpu(), F.linear(x, w)) <= 2e-3
 
 
+@pytest.mark.parametrize("H", [256, 512, 768, 1024, 1536])
+@pytest.mark.parametrize("M", [1, 7, 9, 3601])  # a row, around the 8 groups of a CTA, more rows than one pass of the grid
+def test_norm_row_groups(M, H):
+    test_rms_norm_matches_torch(torch.float32, torch.bfloat16, M, H)
+    test_add_rms_norm_matches_torch(torch.bfloat16, torch.bfloat16, M, H)
+
+
 @pytest.mark.parametrize("W,R,T", [(4, 64, 1), (4, 192, 2), (4, 512, 3), (2, 64, 9), (1, 64, 5)])
 @pytest.mark.parametrize("cache_dtype", [torch.bfloat16, torch.float32])
 def test_core_params_and_cache_store(W, R, T, cache_dtype):
