@@ -274,17 +274,26 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
     const float l = lam[ch0 + threadIdx.x];
     spc[threadIdx.x] = l > 20.f ? l : softplus_f(l);
   }
-  pdl_wait();
-  pdl_trigger();
-
   // A thread owns 8 consecutive channels of one batch row (TB * BW / 8 <= 256 threads have work): every
   // global input arrives as 16-byte loads, all requested before anything waits.
   constexpr int VEC = 8, TPR = BW / VEC;  // threads per batch row
   const int eb = threadIdx.x / TPR, ec = (threadIdx.x % TPR) * VEC;
   const bool has = threadIdx.x < TB * TPR, ok = has && b0 + eb < B;
-  float xn[VEC], yv[VEC], sv[VEC], cacc[VEC], win[3][VEC];
+  float xn[VEC], yv[VEC], sv[VEC], cacc[VEC], win[3][VEC], taps[4][VEC];
 #pragma unroll
-  for (int v = 0; v < VEC; ++v) xn[v] = yv[v] = sv[v] = cacc[v] = win[0][v] = win[1][v] = win[2][v] = 0.f;
+  for (int v = 0; v < VEC; ++v) {
+    xn[v] = yv[v] = sv[v] = cacc[v] = win[0][v] = win[1][v] = win[2][v] = 0.f;
+    taps[0][v] = taps[1][v] = taps[2][v] = taps[3][v] = 0.f;
+  }
+  if (ok) {
+    load_dep8(cb + ch0 + ec, cacc);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < W) load_dep8(cw + (int64_t)j * R + ch0 + ec, taps[j]);
+  }
+  pdl_wait();
+  pdl_trigger();
+
   if (ok) {
     const int64_t bg = b0 + eb;
     const int ch = ch0 + ec;
@@ -296,19 +305,19 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
 #pragma unroll
     for (int j = 0; j < 3; ++j)
       if (j < W - 1) load_dep8(sp + (int64_t)j * R, win[j]);
-    float wv[VEC];
-    VecIO<float, VEC>::load(cb + ch, cacc);
-    VecIO<float, VEC>::load(cw + (int64_t)(W - 1) * R + ch, wv);
+    // state row j is x[t-(W-1)+j], paired with w[j]; the new input with w[W-1]
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) cacc[v] = fmaf(wv[v], xn[v], cacc[v]);
+    for (int j = 0; j < 4; ++j)
+      if (j == W - 1) {
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {  // state row j is x[t-(W-1)+j], paired with w[j]
-      if (j < W - 1) {
-        VecIO<float, VEC>::load(cw + (int64_t)j * R + ch, wv);
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) cacc[v] = fmaf(wv[v], win[j][v], cacc[v]);
+        for (int v = 0; v < VEC; ++v) cacc[v] = fmaf(taps[j][v], xn[v], cacc[v]);
       }
-    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (j < W - 1) {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) cacc[v] = fmaf(taps[j][v], win[j][v], cacc[v]);
+      }
   }
   // conv outputs (rounded to bf16) to shared memory, and the cache roll (hawk/hawk.py:168-179, hawk/cache.py:37-43)
   if (has) VecIO<bf, VEC>::store(xcb + eb * KP + ec, cacc);  // rows past the batch hold zeros

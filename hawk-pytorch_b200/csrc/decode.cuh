@@ -6,16 +6,31 @@
 
 namespace hawk {
 
+// 8 elements from their 16-byte words (one of bf16, two of fp32)
+__device__ __forceinline__ void unpack8(const uint4 (&r)[1], float (&v)[8]) {
+  const float2 q0 = unpack_bf16x2(r[0].x), q1 = unpack_bf16x2(r[0].y), q2 = unpack_bf16x2(r[0].z), q3 = unpack_bf16x2(r[0].w);
+  v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y; v[4] = q2.x; v[5] = q2.y; v[6] = q3.x; v[7] = q3.y;
+}
+__device__ __forceinline__ void unpack8(const uint4 (&r)[2], float (&v)[8]) {
+  v[0] = __uint_as_float(r[0].x); v[1] = __uint_as_float(r[0].y); v[2] = __uint_as_float(r[0].z); v[3] = __uint_as_float(r[0].w);
+  v[4] = __uint_as_float(r[1].x); v[5] = __uint_as_float(r[1].y); v[6] = __uint_as_float(r[1].z); v[7] = __uint_as_float(r[1].w);
+}
+// and back, rounding to the type
+__device__ __forceinline__ void pack8(const float (&v)[8], uint4 (&r)[1]) {
+  r[0] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+__device__ __forceinline__ void pack8(const float (&v)[8], uint4 (&r)[2]) {
+  r[0] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+  r[1] = make_uint4(__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7]));
+}
 // 8 consecutive elements written by the preceding kernel (16-byte aligned), as fp32
 __device__ __forceinline__ void load_dep8(const float* p, float (&v)[8]) {
-  const uint4 a = ld_dep16(p), b = ld_dep16(p + 4);
-  v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
-  v[4] = __uint_as_float(b.x); v[5] = __uint_as_float(b.y); v[6] = __uint_as_float(b.z); v[7] = __uint_as_float(b.w);
+  const uint4 r[2] = {ld_dep16(p), ld_dep16(p + 4)};
+  unpack8(r, v);
 }
 __device__ __forceinline__ void load_dep8(const __nv_bfloat16* p, float (&v)[8]) {
-  const uint4 a = ld_dep16(p);
-  const float2 q0 = unpack_bf16x2(a.x), q1 = unpack_bf16x2(a.y), q2 = unpack_bf16x2(a.z), q3 = unpack_bf16x2(a.w);
-  v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y; v[4] = q2.x; v[5] = q2.y; v[6] = q3.x; v[7] = q3.y;
+  const uint4 r[1] = {ld_dep16(p)};
+  unpack8(r, v);
 }
 // one element of the same
 __device__ __forceinline__ float load_dep(const float* p) { return *static_cast<const volatile float*>(p); }

@@ -21,15 +21,18 @@ using namespace tc;
 //
 // A CTA computes 128 rows of W against a slice of K; the `splits` CTAs of a cluster share a tile and add their partial
 // sums through each other's shared memory in a fixed order (no workspace, no second launch).  The split is what puts a
-// 2048 x 2048 projection (16 tiles) on all SMs; linear_plan() chooses it.  Two CTAs fit an SM (a ring of 2 to 6 stages of
-// 64 K each, 96 to 108 KB; 256 TMEM columns at most), so that the next launch's CTAs load while this one's finish.
+// 2048 x 2048 projection (16 tiles) on all SMs; linear_plan() chooses it.  Two or three CTAs fit an SM (rings of 2 to 4
+// stages of 64 K; 256 TMEM columns at most), so that the next launch's CTAs load while this one's finish.
 //
 // WF32: W is fp32 (a model under autocast) and is rounded to bf16 on its way to shared memory by eight warps, the same
 // rounding that a cast pass makes: 4 bytes of traffic per weight instead of 4 + 2 + 2.
 // GEGLU: W is [gate | up] (2N rows); a tile is 64 gate rows and their 64 up rows and leaves as gelu(gate) * up.
 // ---------------------------------------------------------------------------------------------
 constexpr int DL_ROWS = 128, DL_BK = 64, DL_W_BYTES = DL_ROWS * DL_BK * 2, DL_MAX_STAGES = 6, DL_MAX_SPLITS = 8;
-constexpr int DL_RING = 108 * 1024;  // of the 113 KB per CTA that two CTAs per SM may have
+// Bytes of a CTA's ring.  Up to 64 tokens three CTAs fit an SM, so that the next launch's are there to read its weights early
+// (16 / 64 tokens through 6 layers of 2048: 308 / 353 us against 337 / 378 with rings of 108 KB, of which two fit); more
+// tokens need the larger ring for two stages or three (128 tokens: 448 against 505).
+constexpr int dl_ring(int npad) { return npad <= 64 ? 74 * 1024 : 108 * 1024; }
 
 struct LinearArgs {
   int M, N, K, npad, splits, stages, chunk, early;
@@ -259,7 +262,7 @@ static int linear_launch(const __nv_bfloat16* x, const void* w, int w_dtype, __n
   }
   const int stage = DL_W_BYTES + a.npad * DL_BK * 2;
   a.M = M; a.N = N; a.K = K; a.early = early; a.out = out; a.status = status;
-  a.stages = std::min(DL_MAX_STAGES, DL_RING / stage);
+  a.stages = std::min(DL_MAX_STAGES, dl_ring(a.npad) / stage);
   const int max_chunk = a.stages * stage / (DL_ROWS * 4) / 16 * 16, chunks = (a.npad + max_chunk - 1) / max_chunk;
   a.chunk = ((a.npad + chunks - 1) / chunks + 15) / 16 * 16;
   const int tiles = geglu ? (N + 63) / 64 : (N + DL_ROWS - 1) / DL_ROWS;
@@ -331,18 +334,21 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: groups of 8 tokens; KB: blocks of 32 k per warp and step
-template <typename WT, int NT, int KB, bool GEGLU, int NORM>
-__global__ void __launch_bounds__(256, 2) decode_rows_kernel(RowsArgs p) {
+// NT: groups of 8 tokens; KB: blocks of 32 k per warp and step; WARPS: 8, or 16 where a row of W is so long that eight warps
+// would take it in three steps with one CTA per SM
+template <typename WT, int NT, int KB, int WARPS, bool GEGLU, int NORM>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) decode_rows_kernel(RowsArgs p) {
   using bf = __nv_bfloat16;
   using TX = typename std::conditional<NORM == 2, float, bf>::type;  // storage of x
-  __shared__ float red[2][8][16][8 * NT];
-  __shared__ float stat[8][8 * NT];
+  constexpr int XV = sizeof(TX) / 2;                                  // 16-byte loads per 8 elements of x
+  __shared__ float red[2][WARPS][16][8 * NT];
+  __shared__ float stat[WARPS][8 * NT];
+  extern __shared__ __align__(16) float norm_w[];  // NORM: [K]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-  const int chunks = (p.K + 256 * KB - 1) / (256 * KB);
+  const int chunks = (p.K + 32 * WARPS * KB - 1) / (32 * WARPS * KB);
   const WT* w = static_cast<const WT*>(p.w);
   const TX* x = static_cast<const TX*>(p.x);
-  auto k_of = [&](int c, int j) { return ((c * 8 + warp) * KB + j) * 32 + tig * 8; };
+  auto k_of = [&](int c, int j) { return ((c * WARPS + warp) * KB + j) * 32 + tig * 8; };
 
   WFrag<WT> wf[KB][2];
   auto load_w = [&](int item, int c) {
@@ -361,37 +367,96 @@ __global__ void __launch_bounds__(256, 2) decode_rows_kernel(RowsArgs p) {
   pdl_wait();
   pdl_trigger();
 
-  // the value of x + delta that the norm sees, 8 columns of one row
-  auto sum8 = [&](int tok, int k, float (&v)[8]) {
-    load_dep8(x + (size_t)tok * p.K + k, v);
-    if (p.delta) {
-      float d[8];
-      load_dep8(p.delta + (size_t)tok * p.K + k, d);
+  uint4 xf[NT][KB];
+  float inv[NT];
+  if (NORM) {
+    for (int k = threadIdx.x * 4; k < p.K; k += WARPS * 128) copy_async16(norm_w + k, p.norm_w + k);
+  }
+  // NORM: x + delta of chunk c, as the norm sees it, in x's precision.  All of x and four blocks of delta are requested before
+  // any is used (block by block these loads took 6 of the kernel's 8 us).
+  uint4 xs[NT][NORM ? KB : 1][XV];
+  auto fetch_sum = [&](int c) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = from_float_round<TX>(v[q] + d[q]);
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int j = 0; j < KB; ++j) {
+        const int k = k_of(c, j), tok = t * 8 + gid;
+        const bool ok = k < p.K && tok < p.M;
+#pragma unroll
+        for (int h = 0; h < XV; ++h) xs[t][j][h] = ok ? ld_dep16(x + (size_t)tok * p.K + k + h * 4) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    if (p.delta == nullptr) return;
+    constexpr int STEP = KB < 4 ? KB : 4;
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int j0 = 0; j0 < KB; j0 += STEP) {
+        uint4 dr[STEP][1];
+        const int tok = t * 8 + gid;
+#pragma unroll
+        for (int j = 0; j < STEP; ++j) {
+          const int k = k_of(c, j0 + j);
+          dr[j][0] = k < p.K && tok < p.M ? ld_dep16(p.delta + (size_t)tok * p.K + k) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int j = 0; j < STEP; ++j) {
+          float v[8], d[8];
+          unpack8(xs[t][j0 + j], v);
+          unpack8(dr[j], d);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] += d[q];
+          pack8(v, xs[t][j0 + j]);
+        }
+      }
+  };
+  auto normalise = [&](int c) {
+#pragma unroll
+    for (int j = 0; j < KB; ++j) {
+      const int k = k_of(c, j);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        float v[8];
+        unpack8(xs[t][j], v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = k < p.K ? (v[q] * inv[t]) * norm_w[k + q] : 0.f;
+        uint4 o[1];
+        pack8(v, o);
+        xf[t][j] = o[0];
+      }
     }
   };
-  float inv[NT];
+  auto load_x = [&](int c) {
+    if (NORM) {
+      fetch_sum(c);
+      normalise(c);
+    } else {
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int j = 0; j < KB; ++j) {
+          const int k = k_of(c, j), tok = t * 8 + gid;
+          xf[t][j] = k < p.K && tok < p.M ? ld_dep16(x + (size_t)tok * p.K + k) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+  };
   if (NORM) {
     float ss[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) ss[t] = 0.f;
     for (int c = 0; c < chunks; ++c) {
+      fetch_sum(c);
 #pragma unroll
-      for (int j = 0; j < KB; ++j) {
-        const int k = k_of(c, j);
+      for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const int tok = t * 8 + gid;
-          if (k < p.K && tok < p.M) {
-            float v[8];
-            sum8(tok, k, v);
-            if (p.delta && blockIdx.x == 0) VecIO<TX, 8>::store(static_cast<TX*>(p.x_out) + (size_t)tok * p.K + k, v);
+        for (int j = 0; j < KB; ++j) {
+          const int k = k_of(c, j), tok = t * 8 + gid;
+          float v[8];
+          unpack8(xs[t][j], v);
+          if (p.delta && blockIdx.x == 0 && k < p.K && tok < p.M)
+            VecIO<TX, 8>::store(static_cast<TX*>(p.x_out) + (size_t)tok * p.K + k, v);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) ss[t] = fmaf(v[q], v[q], ss[t]);
-          }
+          for (int q = 0; q < 8; ++q) ss[t] = fmaf(v[q], v[q], ss[t]);
         }
-      }
     }
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
@@ -399,41 +464,20 @@ __global__ void __launch_bounds__(256, 2) decode_rows_kernel(RowsArgs p) {
       ss[t] += __shfl_xor_sync(0xffffffffu, ss[t], 2);
       if (tig == 0) stat[warp][t * 8 + gid] = ss[t];
     }
+    copy_async_wait();
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
       float s = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) s += stat[k][t * 8 + gid];
+      for (int k = 0; k < WARPS; ++k) s += stat[k][t * 8 + gid];
       inv[t] = rsqrtf(s / (float)p.K + p.eps);
     }
+    if (chunks > 1) fetch_sum(0);
+    normalise(0);
+  } else {
+    load_x(0);
   }
-  uint4 xf[NT][KB];
-  auto load_x = [&](int c) {
-#pragma unroll
-    for (int j = 0; j < KB; ++j) {
-      const int k = k_of(c, j);
-      float nw[8];
-      if (NORM && k < p.K) load_dep8(p.norm_w + k, nw);
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const int tok = t * 8 + gid;
-        xf[t][j] = make_uint4(0u, 0u, 0u, 0u);
-        if (k < p.K && tok < p.M) {
-          if (NORM) {
-            float v[8];
-            sum8(tok, k, v);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] = (v[q] * inv[t]) * nw[q];
-            xf[t][j] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-          } else {
-            xf[t][j] = ld_dep16(x + (size_t)tok * p.K + k);
-          }
-        }
-      }
-    }
-  };
-  load_x(0);
 
   int par = 0;
   for (; item < p.items; item += gridDim.x, par ^= 1) {
@@ -467,7 +511,7 @@ __global__ void __launch_bounds__(256, 2) decode_rows_kernel(RowsArgs p) {
       if (tok < p.M && tok < 8 * NT && col < p.N) {
         float g = 0.f, u = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < WARPS; ++k) {
           g += red[par][k][j][tok];
           u += red[par][k][j + 8][tok];
         }
@@ -480,7 +524,7 @@ __global__ void __launch_bounds__(256, 2) decode_rows_kernel(RowsArgs p) {
       if (tok < p.M && tok < 8 * NT && col < p.N) {
         float s = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) s += red[par][k][r][tok];
+        for (int k = 0; k < WARPS; ++k) s += red[par][k][r][tok];
         p.out[(size_t)tok * p.N + col] = __float2bfloat16(s);
       }
     }
@@ -503,21 +547,27 @@ static int rows_launch(int norm, const void* x, const void* delta, void* x_out, 
   const dim3 grid((unsigned)std::min(a.items, 2 * sm_count()));
   // The widest step that the registers hold (128 per thread: 8 blocks of 32 bf16 weights in two rows are 64 of them), and no
   // wider than the eight warps need for all of K.
-#define HAWK_ROWS(WT, NT, KB, G, NM) return launch_kernel(decode_rows_kernel<WT, NT, KB, G, NM>, grid, dim3(256), 0, st, true, 1, a)
-#define HAWK_ROWS_KB(G, NM)                                   \
-  do {                                                        \
-    if (w_dtype == HAWK_BF16) {                               \
-      if (M > 8) {                                            \
-        if (K <= 512) HAWK_ROWS(__nv_bfloat16, 2, 2, G, NM);  \
-        HAWK_ROWS(__nv_bfloat16, 2, 4, G, NM);                \
-      }                                                       \
-      if (K <= 512) HAWK_ROWS(__nv_bfloat16, 1, 2, G, NM);    \
-      if (K <= 1024) HAWK_ROWS(__nv_bfloat16, 1, 4, G, NM);   \
-      HAWK_ROWS(__nv_bfloat16, 1, 8, G, NM);                  \
-    }                                                         \
-    if (M > 8) HAWK_ROWS(float, 2, 2, G, NM);                 \
-    if (K <= 512) HAWK_ROWS(float, 1, 2, G, NM);              \
-    HAWK_ROWS(float, 1, 4, G, NM);                            \
+  const size_t smem = norm ? (size_t)K * 4 : 0;
+#define HAWK_ROWS(WT, NT, KB, WARPS, G, NM) \
+  return launch_kernel(decode_rows_kernel<WT, NT, KB, WARPS, G, NM>, grid, dim3(WARPS * 32), smem, st, true, 1, a)
+#define HAWK_ROWS_KB(G, NM)                                                        \
+  do {                                                                             \
+    if (w_dtype == HAWK_BF16) {                                                    \
+      if (M > 8) {                                                                 \
+        if (K <= 512 || NM == 2) HAWK_ROWS(__nv_bfloat16, 2, 2, 8, G, NM);         \
+        HAWK_ROWS(__nv_bfloat16, 2, 4, 8, G, NM);                                  \
+      }                                                                            \
+      if (K <= 512) HAWK_ROWS(__nv_bfloat16, 1, 2, 8, G, NM);                      \
+      if (K <= 1024 || NM == 2) HAWK_ROWS(__nv_bfloat16, 1, 4, 8, G, NM);          \
+      if constexpr (NM == 0 && !G)                                                 \
+        if (K > 2048 && a.items <= sm_count()) HAWK_ROWS(__nv_bfloat16, 1, 8, 16, G, NM); \
+      if constexpr (NM != 2) HAWK_ROWS(__nv_bfloat16, 1, 8, 8, G, NM);             \
+    }                                                                              \
+    if (M > 8) HAWK_ROWS(float, 2, 2, 8, G, NM);                                   \
+    if (K <= 512) HAWK_ROWS(float, 1, 2, 8, G, NM);                                \
+    if constexpr (NM == 0 && !G)                                                   \
+      if (K > 1024 && a.items <= sm_count()) HAWK_ROWS(float, 1, 4, 16, G, NM);    \
+    HAWK_ROWS(float, 1, 4, 8, G, NM);                                              \
   } while (0)
   if (geglu) {
     if (norm == 1) HAWK_ROWS_KB(true, 1);
