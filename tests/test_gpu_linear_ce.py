@@ -146,3 +146,24 @@ def test_backward_as_a_threads_first_cuda_call():
     t.start()
     t.join()
     assert len(got) == 2 and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+# tile heights and K splits that plan_grad chooses: one K block and one ragged pair tile; many splits of a ragged tile; two
+# halves per pair with and without splits, both ragged, in either gradient; mixed operand types
+@pytest.mark.parametrize("N,H,V", [(1, 8, 2), (255, 72, 257), (513, 264, 1031), (300, 72, 5000), (4000, 520, 9000)])
+@pytest.mark.parametrize("wdt,adt", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+def test_linear_ce_tiles_and_splits(N, H, V, wdt, adt):
+    from hawk_b200 import check_device_status, fused_cross_entropy
+    g = torch.Generator(device="cuda").manual_seed(N + V)
+    w = (torch.randn(V, H, generator=g, device="cuda") / math.sqrt(H)).bfloat16()
+    act = torch.randn(N, H, generator=g, device="cuda").bfloat16()
+    labels = torch.randint(0, V, (N,), generator=g, device="cuda")
+    wd, ad = w.to(wdt).requires_grad_(), act.to(adt).requires_grad_()
+    loss = fused_cross_entropy(wd, ad, labels)
+    (1.7 * loss).backward()
+    check_device_status()
+    w64, a64 = w.detach().double().requires_grad_(), act.detach().double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(a64 @ w64.t(), labels)
+    (1.7 * ref).backward()
+    assert wd.grad.dtype == wdt and ad.grad.dtype == adt and abs(float(loss) - float(ref)) <= TOL * float(ref)
+    assert rel_l2(wd.grad, w64.grad) <= TOL and rel_l2(ad.grad, a64.grad) <= TOL
