@@ -859,30 +859,49 @@ static int launch_bwd(const void* x, const void* gx, const void* ga, const float
 
 // Launch shape.  A CTA scans all of T for its channel group, so the grid is B * D / CW CTAs of equal cost and what matters is
 // how evenly they fill the 148 SMs and how many rows are in flight on each.  Measured on B200, bf16, L2 flushed, us (R rows
-// per slot x warps x CW):
-//   plain forward                        8x4x32   8x8x32   16x4x16   (before: 8x4x16 / 8x8x16)
-//     B16 T4096 D2048  (1024 groups of 32)  187      195       232      236
-//     B8  T4096 D2048   (512)               109      116       128      126
-//     B16 T2048 D512    (256)                45       38        48       53
-//     B5  T3001 D1536   (240)                59       50        58       62
-//     B1  T65536 D4096  (128)               793      568       507      523
-//     B2  T16384 D2048  (128)               207      151       139      144
-//     B1  T16384 D1024 and other few groups: as 16x4x16, or the time split below
+// per slot x warps x CW; the lists of shapes tried are longer):
+//   plain forward                          8x4x32   8x8x32   16x8x32   16x4x16   8x8x16
+//     B16 T4096 D2048  (1024 groups of 32)    187      195                 232      264
+//     B8  T4096 D2048   (512)                 109      116                 128      144
+//     B16 T2048 D512    (256)                  45       38                  48       53
+//     B5  T3001 D1536   (240)                  59       50        59        57       62
+//     B1  T65536 D4096  (128)                 793      568       508       508      523
+//     B2  T16384 D2048  (128)                 207      151       135       139      144
+//     B8  T2048 D512    (128)                  35       28        25        29       31
+//     B4  T2000 D768     (96)                  34       26        25        25       28
 //   so: 4 warps of CW = 32 where 400 or more CTAs come of it (four fit an SM), 8 warps of CW = 32 where they still reach
-//   every SM, else CW = 16 with 16 rows per slot.
-//   plain backward                       8x8x64   8x8x32   8x16x32
-//     B8  T4096 D2048                       204      216       239
-//     B5  T3001 D1536                        89       89        99
-//     B1  T65536 D4096                     1629      968       884   (fused epilogue: 1250 -> 1164)
-//     B2  T16384 D2048                      417      253       233   (fused epilogue:  323 ->  302)
-//     B4  T2000 D768     (96)                63       44        42   (fused epilogue:   52 ->   54)
-//   so: CW = 64 with 8 warps from 200 of its groups on, CW = 32 below; one CTA of 16 warps instead of one of 8 where there is
-//   at most one per SM and the sequence is long enough for the larger super-steps.
+//   every SM, with 16 rows per slot where there is one CTA per SM at most, else (few groups, short sequences) CW = 16.
+//   plain backward                         8x8x64   8x8x32   16x8x32   8x16x32
+//     B8  T4096 D2048                         204      216                 239
+//     B5  T3001 D1536                          89       89        99       101
+//     B1  T65536 D4096                       1629      970       855       886
+//     B2  T16384 D2048                        417      253       226       233
+//     B4  T2000 D768                           63       44        42        42
+//   so: CW = 64 with 8 warps from 200 of its groups on, else CW = 32, with 16 rows per slot where there is one CTA per SM.
+//   With the fused epilogue, one CTA per SM (before: 8x8x32): forward 16x8x32 B1 T65536 D4096 751 -> 688, B2 T16384 D2048
+//   196 -> 180; backward 8x12x32 1252 -> 1121 and 323 -> 292, B8 T2048 D512 52 -> 50 (16x8x32: 1152, 300, 52).
 // The fused-epilogue kernels carry more arithmetic per byte: CW = 32 in the forward throughout (inside the training step
 // 186 against 224 us for CW = 16, at B8 T4096 D2048), otherwise the same lines.
+// fp32 storage (IEEE division, expf, sqrtf: more instructions per element, so more warps pay), us:
+//   plain forward                          4x4x16 (before)   4x8x16   8x8x16
+//     B8  T4096 D2048  (512 groups of 32)       311            246      309
+//     B5  T3001 D1536  (240)                    131            116      132
+//     B16 T2048 D512   (256)                     92             82       92
+//     B1  T32768 D4096 (128)                   1071            676      643
+//     B1  T65536 D2048  (64)                   1948           1126     1070
+//   plain backward                         2x8x64 / 2x8x32 (before)   4x8x32   4x16x32   8x8x16
+//     B8  T4096 D2048                           489                    458       480      648
+//     B5  T3001 D1536                           192                    179       189      284
+//     B1  T32768 D4096                         1529                   1385       927     1412
+//     B8  T2048 D512   (128)                    107                     99        73      106
+//     B1  T65536 D2048                         3043                   2755      1840     1420
+//     B3  T517 D512     (48)                     38                     36        30       28
+//   The lines are those of the bf16 kernels: whether CTAs of 32 channels reach every SM, or at least half of them.
 static bool many_groups(int B, int D) { return (int64_t)B * (D / 64) >= 200; }
 static int64_t groups32(int B, int D) { return (int64_t)B * (D / 32); }
 constexpr int kSms = 148;
+// at most one CTA of 32 channels per SM, on more than half of them, and enough rows for super-steps of 192 to 256
+static bool one_cta_per_sm(int B, int T, int D) { return groups32(B, D) > kSms / 2 && groups32(B, D) <= kSms && T >= 1024; }
 
 static int check_scan_common(int B, int T, int D, int dtype) {
   HAWK_REQUIRE(valid_dtype(dtype), HAWK_ERR_DTYPE);
@@ -915,18 +934,21 @@ static int scan_fwd_dispatch(const void* x, const void* gx, const void* ga, cons
   }
 #define HAWK_FWD(TT, R, W, LPR, S, MINB, FAST, GELU) \
   return launch_fwd<TT, R, W, LPR, S, MINB, FAST, GELU>(x, gx, ga, lam, h0, gate_bias, h, B, T, D, ge ? *ge : none, st)
-  const bool many = many_groups(B, D);
+  const bool many = many_groups(B, D), one_per_sm = one_cta_per_sm(B, T, D);
   if (dtype == HAWK_BF16) {
     if (ge) {
       if (many) HAWK_FWD(bf, 8, 4, 16, 2, 4, true, true);
+      if (one_per_sm) HAWK_FWD(bf, 16, 8, 16, 2, 1, true, true);
       HAWK_FWD(bf, 8, 8, 16, 2, 2, true, true);
     }
     if (many) HAWK_FWD(bf, 8, 4, 16, 2, 4, true, false);
     if (groups32(B, D) > kSms) HAWK_FWD(bf, 8, 8, 16, 2, 2, true, false);
+    if (one_per_sm) HAWK_FWD(bf, 16, 8, 16, 2, 1, true, false);
     HAWK_FWD(bf, 16, 4, 8, 2, 4, true, false);
   }
   if (ge) HAWK_FWD(float, 4, 4, 8, 4, 3, false, true);
-  HAWK_FWD(float, 4, 4, 8, 4, 4, false, false);
+  if (groups32(B, D) <= kSms) HAWK_FWD(float, 8, 8, 8, 2, 2, false, false);
+  HAWK_FWD(float, 4, 8, 8, 2, 4, false, false);
 #undef HAWK_FWD
 }
 
@@ -955,23 +977,24 @@ static int scan_bwd_dispatch(const void* x, const void* gx, const void* ga, cons
   return launch_bwd<TT, R, W, LPR, S, MINB, FAST, GELU>(x, gx, ga, lam, h0, gate_bias, h, go, dx, dgx, dga, dlam, dh0, \
                                                         dgate_bias, partial, B, T, D, ge ? *ge : none, st,            \
                                                         split ? *split : whole)
-  const bool many = many_groups(B, D), one_per_sm = groups32(B, D) > kSms / 2 && groups32(B, D) <= kSms;
+  const bool many = many_groups(B, D), one_per_sm = one_cta_per_sm(B, T, D);
   if (dtype == HAWK_BF16) {
     if (ge) {
       if (many) HAWK_BWD(bf, 8, 8, 32, 2, 2, true, true);
-      if (one_per_sm && T >= 4096) HAWK_BWD(bf, 8, 16, 16, 2, 1, true, true);
+      if (one_per_sm) HAWK_BWD(bf, 8, 12, 16, 2, 1, true, true);
       HAWK_BWD(bf, 8, 8, 16, 2, 2, true, true);
     }
     if (many) HAWK_BWD(bf, 8, 8, 32, 2, 2, true, false);
-    if (one_per_sm && T >= 4096) HAWK_BWD(bf, 8, 16, 16, 2, 1, true, false);
+    if (one_per_sm) HAWK_BWD(bf, 16, 8, 16, 2, 1, true, false);
     HAWK_BWD(bf, 8, 8, 16, 2, 2, true, false);
   }
   if (ge) {
     if (many) HAWK_BWD(float, 2, 8, 32, 4, 2, false, true);
     HAWK_BWD(float, 2, 8, 16, 4, 2, false, true);
   }
-  if (many) HAWK_BWD(float, 2, 8, 32, 4, 2, false, false);
-  HAWK_BWD(float, 2, 8, 16, 4, 2, false, false);
+  if (groups32(B, D) > kSms) HAWK_BWD(float, 4, 8, 16, 2, 2, false, false);
+  if (groups32(B, D) > kSms / 2) HAWK_BWD(float, 4, 16, 16, 2, 1, false, false);
+  HAWK_BWD(float, 8, 8, 8, 2, 2, false, false);
 #undef HAWK_BWD
 }
 

@@ -298,9 +298,16 @@ def test_reference_host_function_names():
 
 
 # one shape per line of the launch rule, with ragged last super-steps: CTAs of 32 channels past 400, between 148 and 400, and
-# at most 148 with a long sequence (16-row slots of 16 channels forward, 16 warps backward)
+# at most 148 with a long sequence (16-row slots)
 @pytest.mark.parametrize("B,T,D", [(25, 67, 512), (10, 131, 512), (10, 257, 512), (1, 4097, 2560), (3, 4355, 1024)])
 def test_scan_bf16_launch_shapes(B, T, D):
     x, gx, ga, go, lam = _inputs(B, T, D, seed=11 + T, dtype=torch.bfloat16)
     got = _run_gpu(x, gx, ga, go, lam, torch.bfloat16)
     _check(got, _oracle(x, gx, ga, go, lam, got[0]), BF16_TOL)
+
+
+@pytest.mark.parametrize("B,T,D", [(10, 131, 512), (10, 257, 512), (1, 1025, 2560), (3, 259, 1024)])
+def test_scan_fp32_launch_shapes(B, T, D):
+    x, gx, ga, go, lam = _inputs(B, T, D, seed=13 + T)
+    got = _run_gpu(x, gx, ga, go, lam, torch.float32)
+    _check(got, _oracle(x, gx, ga, go, lam, got[0]), FP32_TOL)

@@ -121,7 +121,7 @@ def test_fused_scan_gelu_metric_shape_properties():
 
 
 def test_long_sequence_of_few_groups():
-    """The 16-warp backward (80 groups of 32 channels, over 4096 rows), with a ragged last super-step."""
+    """One CTA per SM (80 groups of 32 channels): 16-row slots forward, 12 warps backward, ragged last super-steps."""
     args = _inputs(1, 4099, 2560, 5, torch.bfloat16)
     got = _run(*args, torch.bfloat16, True)
     x, gx, ga, dout, xy, gb, lam = args
