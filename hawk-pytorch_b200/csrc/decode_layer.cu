@@ -532,9 +532,9 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) decode_rows_kernel(Row
 }
 
 // decode_rows_kernel or the tensor-core kernel above: 8 tokens or fewer always; up to 16 where a CTA's registers hold the
-// whole of a row of W beside two groups of tokens.  One token through 24 layers of width 2048 and the head (bf16) takes 1062
-// us, 1108 with the other kernel; 16 tokens through 8 layers of width 512 (fp32 weights) 183 against 252, but through 6 of
-// width 1024 227 against 215 and of width 2048 702 against 345: there x is read again for every 16 rows of W.
+// whole of a row of W beside two groups of tokens.  One token through 6 layers of width 2048 and the head (bf16) takes 229 us,
+// 316 with the other kernel; 16 tokens through 8 layers of width 512 (fp32 weights) 153 against 252.  16 tokens of width 1024
+// and 2048 take 246 and 421 us with their x in shared memory (every CTA reads all of it) against 212 and 310.
 static bool few_rows(int M, int width) { return M <= 8 || (M <= 16 && width <= 512); }
 
 // norm: 0 x is bf16 and multiplied as it is; 1 / 2: the residual in bf16 / fp32

@@ -320,14 +320,13 @@ def _chain_weight(layer: nn.Linear, autocast: bool) -> Optional[torch.Tensor]:
     return w if w.dtype == torch.bfloat16 else None
 
 
-def chain_rows(hidden_size: int, fp32_weights: bool) -> int:
+def chain_rows(fp32_weights: bool) -> int:
     """Up to how many sequences the chained kernels beat the modules called one by one.  Measured on B200, us per token, chain
-    against modules: 6 layers of 2048 in bf16 273 / 377 at 1 sequence, 292 / 371 at 8, 349 / 331 at 32; 6 layers of 1024
-    215 / 227 at 32, 236 / 224 at 64; fp32 weights (which the modules cast on every call) 8 layers of 512 123 / 311 at 1,
-    279 / 321 at 64, 342 / 328 at 128; 4 layers of 2048 487 / 527 at 64, 555 / 536 at 128."""
-    if fp32_weights:
-        return 64
-    return 32 if hidden_size <= 1024 else 8
+    against modules: 6 layers of 2048 in bf16 232 / 391 at 1 sequence, 242 / 382 at 8, 310 / 343 at 16, 326 / 336 at 32, 355 /
+    340 at 64; 6 layers of 1024 109 / 255 at 1, 218 / 237 at 32, 244 / 231 at 64; fp32 weights (which the modules cast on every
+    call) 8 layers of 512 114 / 314 at 1, 268 / 326 at 64, 340 / 335 at 128; 4 layers of 2048 433 / 526 at 64, 551 / 517 at
+    128."""
+    return 64 if fp32_weights else 32
 
 
 def _chain_ok(hidden: torch.Tensor) -> Optional[bool]:
@@ -383,12 +382,14 @@ class RNNLayer(nn.Module):
             return None
         weights = [_chain_weight(m, autocast) for m in linears]
         state = cache.recc_state
+        B, R = residual.shape[0], gi.width
         if (any(w is None or w.device != residual.device for w in weights)
-                or residual.shape[0] > chain_rows(residual.shape[2], all(w.dtype == torch.float32 for w in weights)) or gi.block_width > 128 or conv.temporal_width > 4
-                or gi.width % 8 or weights[3].shape[1] % 8 or gi.w.dtype != ga.w.dtype
+                or B > chain_rows(all(w.dtype == torch.float32 for w in weights)) or gi.block_width > 128
+                or conv.temporal_width > 4 or R % 8 or weights[3].shape[1] % 8 or gi.w.dtype != ga.w.dtype
                 or gi.w.dtype not in (torch.float32, torch.bfloat16) or not state.is_contiguous()
                 or not cache.conv_state.is_contiguous() or state.dtype != cache.conv_state.dtype
-                or state.dtype not in (torch.float32, torch.bfloat16) or state.shape[0] != residual.shape[0]):
+                or state.dtype not in (torch.float32, torch.bfloat16) or state.shape != (B, 1, R)
+                or cache.conv_state.shape != (B, conv.temporal_width - 1, R)):
             return None
         out = ops.decode_layer(residual, pending, self.input_norm._weight32(), self.input_norm.eps, weights[0],
                                recc._fp32("w", conv.w), recc._fp32("b", conv.b), gi.w, ga.w, recc._fp32("bx", gi.b),
@@ -439,7 +440,7 @@ class HawkModel(nn.Module):
             if autocast is not None and _plain(self.norm, RMSNorm) and _plain(self.lm_head, nn.Linear):
                 w = _chain_weight(self.lm_head, autocast)
                 if (w is not None and w.shape[0] % 8 == 0 and w.device == hidden.device
-                        and hidden.shape[0] <= chain_rows(hidden.shape[2], w.dtype == torch.float32)):
+                        and hidden.shape[0] <= chain_rows(w.dtype == torch.float32)):
                     return ops.decode_norm_linear(hidden, pending, self.norm._weight32(), self.norm.eps, w, chained), caches
         _, hidden = self.norm.add_forward(hidden, pending)
         if self.use_cache:

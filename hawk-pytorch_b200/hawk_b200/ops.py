@@ -727,10 +727,12 @@ def decode_layer(residual: torch.Tensor, pending: Optional[torch.Tensor], norm1:
     assert w_xy.shape == (2 * R, H) and w_res.shape == (H, R) and w_gu.shape == (2 * I, H) and w_down.shape == (H, I)
     assert nb * bw == R and wx.dtype == wa.dtype and (pending is None or pending.dtype == torch.bfloat16)
     assert conv_state.is_contiguous() and state.is_contiguous() and state.numel() == B * R and conv_state.dtype == state.dtype
+    assert conv_w.shape[1] == R and conv_state.shape == (B, conv_w.shape[0] - 1, R)
     residual = _dense16(residual)
     pending = None if pending is None else _dense16(pending)
     keep = [_dense16(t) for t in (norm1, w_xy, conv_w, conv_b, wx, wa, bx, ba, lam, w_res, norm2, w_gu, w_down)]
     n1, wxy, cw, cb, kx, ka, vx, va, lm, wr, n2, wg, wd = keep
+    follows_layer = follows_layer and wxy.data_ptr() == w_xy.data_ptr()  # not behind a copy just made of it
     out_res = torch.empty_like(residual)
     out_pending = torch.empty(residual.shape, dtype=torch.bfloat16, device=residual.device)
     ws = torch.empty(lib.hawk_decode_layer_workspace_bytes(B, H, R, I, _dt(residual)), dtype=torch.uint8, device=residual.device)
@@ -763,6 +765,7 @@ def decode_norm_linear(residual: torch.Tensor, pending: Optional[torch.Tensor], 
     H, N = residual.shape[-1], weight.shape[0]
     B = residual.numel() // H
     assert weight.shape == (N, H) and (pending is None or pending.dtype == torch.bfloat16)
+    follows_layer = follows_layer and weight.is_contiguous() and weight.data_ptr() % 16 == 0  # not behind a copy of it
     residual, norm, weight = _dense16(residual), _dense16(norm), _dense16(weight)
     pending = None if pending is None else _dense16(pending)
     out = torch.empty(*residual.shape[:-1], N, dtype=torch.bfloat16, device=residual.device)

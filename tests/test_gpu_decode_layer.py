@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 # more than one of its reduction passes (two of 128), the most
 # (H, N): one K block and one tile; K not a multiple of 64 with a ragged tile; every K split up to 8; more tiles than SMs
 @pytest.mark.parametrize("rows", [1, 8, 11, 16, 17, 129, 256])
-@pytest.mark.parametrize("H,N", [(64, 8), (72, 136), (520, 200), (1536, 768), (2048, 20000)])
+@pytest.mark.parametrize("H,N", [(64, 8), (72, 136), (520, 200), (1000, 264), (1536, 768), (2048, 20000)])
 @pytest.mark.parametrize("wdt,rdt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
 def test_norm_linear(rows, H, N, wdt, rdt):
     torch.manual_seed(rows + H + N)
@@ -46,7 +46,8 @@ def _model(vocab, hidden, inter, layers, blocks):
 
 CASES = [(64, 72, 4, b, half) for b in (1, 13, 19, 32) for half in (True, False)]
 CASES += [(256, 768, 16, b, half) for b in (1, 13, 19, 32) for half in (True, False)]
-CASES += [(2048, 6144, 16, b, True) for b in (1, 8)] + [(2048, 6144, 16, b, False) for b in (1, 13, 64)]
+CASES += [(2048, 6144, 16, b, True) for b in (1, 8, 16, 32)] + [(2048, 6144, 16, b, False) for b in (1, 13, 64)]
+CASES += [(1024, 3072, 16, b, True) for b in (2, 11)]
 
 
 @pytest.mark.parametrize("hidden,inter,blocks,batch,half", CASES)
