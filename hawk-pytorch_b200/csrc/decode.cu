@@ -285,6 +285,14 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
     xn[v] = yv[v] = sv[v] = cacc[v] = win[0][v] = win[1][v] = win[2][v] = 0.f;
     taps[0][v] = taps[1][v] = taps[2][v] = taps[3][v] = 0.f;
   }
+  constexpr int KS = BW / 16, NT = 2 * BW / 8, TPW = (NT + 7) / 8;  // k steps, tiles of 8 outputs, tiles per warp
+  const int gid = lane >> 2, tig = lane & 3;
+  float2 bias[TPW];
+#pragma unroll
+  for (int q = 0; q < TPW; ++q) {
+    const int o = (warp + q * 8) * 8;  // output column over both gates
+    bias[q] = o < 2 * BW ? *reinterpret_cast<const float2*>((o < BW ? bx + o : ba + o - BW) + ch0 + 2 * tig) : make_float2(0.f, 0.f);
+  }
   if (ok) {
     load_dep8(cb + ch0 + ec, cacc);
 #pragma unroll
@@ -333,7 +341,6 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
 
   // both gate projections: g[gate][b][j] = bias[j] + sum_k xc[b][k] w[gate][k][j]  (external.py:224-233)
   {
-    constexpr int KS = BW / 16, NT = 2 * BW / 8;
     uint32_t afrag[KS][4];
     const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(xcb + (lane & 15) * KP + (lane >> 4) * 8);
 #pragma unroll
@@ -341,25 +348,35 @@ decode_block_step_mma_kernel(const __nv_bfloat16* __restrict__ xy, int64_t ld_xy
       asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                    : "=r"(afrag[ks][0]), "=r"(afrag[ks][1]), "=r"(afrag[ks][2]), "=r"(afrag[ks][3])
                    : "r"(a_addr + ks * 32));
-    const int gid = lane >> 2, tig = lane & 3;
-    for (int t = warp; t < NT; t += 8) {
-      const int gate = (t * 8) / BW, n0 = t * 8 - gate * BW;
-      const uint32_t b_addr = (uint32_t)__cvta_generic_to_shared(ws + (gate * BW + (lane & 15)) * KP + n0);
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
+    // the warp's TPW tiles side by side: one after the other, each with its own chain of KS MMAs and its bias fetched at the
+    // end, they were 2 of the launch's 9 us
+    float c[TPW][4];
 #pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        uint32_t b0r, b1r;
-        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
-                     : "=r"(b0r), "=r"(b1r)
-                     : "r"(b_addr + ks * 16 * KP * 2));
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                     : "r"(afrag[ks][0]), "r"(afrag[ks][1]), "r"(afrag[ks][2]), "r"(afrag[ks][3]), "r"(b0r), "r"(b1r));
+    for (int q = 0; q < TPW; ++q) c[q][0] = c[q][1] = c[q][2] = c[q][3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+      for (int q = 0; q < TPW; ++q) {
+        const int t = warp + q * 8, gate = (t * 8) / BW, n0 = t * 8 - gate * BW;
+        if (t < NT) {  // the same for the whole warp
+          const uint32_t b_addr = (uint32_t)__cvta_generic_to_shared(ws + (gate * BW + (lane & 15)) * KP + n0);
+          uint32_t b0r, b1r;
+          asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                       : "=r"(b0r), "=r"(b1r)
+                       : "r"(b_addr + ks * 16 * KP * 2));
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                       : "+f"(c[q][0]), "+f"(c[q][1]), "+f"(c[q][2]), "+f"(c[q][3])
+                       : "r"(afrag[ks][0]), "r"(afrag[ks][1]), "r"(afrag[ks][2]), "r"(afrag[ks][3]), "r"(b0r), "r"(b1r));
+        }
       }
-      const float2 bias = *reinterpret_cast<const float2*>((gate ? ba : bx) + ch0 + n0 + 2 * tig);
-      float* gp = g + ((size_t)gate * TB + gid) * BW + n0 + 2 * tig;
-      *reinterpret_cast<float2*>(gp) = make_float2(c[0] + bias.x, c[1] + bias.y);
-      *reinterpret_cast<float2*>(gp + 8 * BW) = make_float2(c[2] + bias.x, c[3] + bias.y);
+#pragma unroll
+    for (int q = 0; q < TPW; ++q) {
+      const int t = warp + q * 8, gate = (t * 8) / BW, n0 = t * 8 - gate * BW;
+      if (t < NT) {
+        float* gp = g + ((size_t)gate * TB + gid) * BW + n0 + 2 * tig;
+        *reinterpret_cast<float2*>(gp) = make_float2(c[q][0] + bias[q].x, c[q][1] + bias[q].y);
+        *reinterpret_cast<float2*>(gp + 8 * BW) = make_float2(c[q][2] + bias[q].x, c[q][3] + bias[q].y);
+      }
     }
   }
   __syncthreads();
