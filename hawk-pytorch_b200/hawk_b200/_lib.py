@@ -51,6 +51,7 @@ SIGNATURES = {
     "hawk_decode_conv_step": (c_int, [_P, c_int64, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P]),
     "hawk_decode_rglru_step": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "hawk_decode_block_step": (c_int, [_P, c_int64] + [_P] * 10 + [c_int] * 7 + [_P]),
+    "hawk_rows_cut": (c_int, [_P, _P, c_int64, c_int, c_int64, c_int, _P]),
     "hawk_core_params": (c_int, [_P, c_int] * 5 + [_P, c_int, c_int, _P]),
     "hawk_cache_store": (c_int, [_P, c_int64, c_int64, _P, _P, _P] + [c_int] * 6 + [_P]),
     "hawk_decode_layer_workspace_bytes": (c_size_t, [c_int] * 5),

@@ -448,7 +448,11 @@ class HawkModel(nn.Module):
         if labels is None:
             return self.lm_head(hidden)
         # next-token loss: position t predicts token t+1 (hawk/hawk.py:291-300)
-        act = hidden[..., :-1, :].reshape(-1, hidden.shape[-1])
+        if (hidden.is_cuda and hidden.dim() == 3 and hidden.shape[1] >= 2 and hidden.numel() and hidden.is_contiguous()
+                and hidden.shape[2] * hidden.element_size() % 16 == 0 and not torch.compiler.is_compiling()):
+            act = ops.drop_last(hidden).view(-1, hidden.shape[-1])
+        else:
+            act = hidden[..., :-1, :].reshape(-1, hidden.shape[-1])
         targets = labels[..., 1:].reshape(-1)
         return ops.fused_cross_entropy(self.lm_head.weight, act, targets)
 

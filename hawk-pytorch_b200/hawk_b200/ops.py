@@ -807,6 +807,43 @@ def check_device_status(device=None) -> None:
             raise RuntimeError("hawk_b200: a tcgen05 GEMM abandoned a bounded mbarrier wait; results are invalid")
 
 
+def _rows_cut(x: torch.Tensor, T: int, cut: int, out: torch.Tensor) -> torch.Tensor:
+    lib = _lib.load()
+    x = _dense16(x)
+    with _on(x, "rows_cut", 1):
+        _lib.check(lib.hawk_rows_cut(x.data_ptr(), out.data_ptr(), x.shape[0], T, x.shape[-1] * x.element_size(), cut, _stream(x)),
+                   "hawk_rows_cut")
+    return out
+
+
+@_operator("hawk_b200::drop_last", mutates_args=())
+def drop_last(x: torch.Tensor) -> torch.Tensor:
+    """x [B,T,H] without its last position, contiguous (H elements a multiple of 16 bytes, T >= 2)."""
+    B, T, H = x.shape
+    return _rows_cut(x, T, 1, torch.empty(B, T - 1, H, dtype=x.dtype, device=x.device))
+
+
+@drop_last.register_fake
+def _(x):
+    return x.new_empty(x.shape[0], x.shape[1] - 1, x.shape[2])
+
+
+@_operator("hawk_b200::append_zero", mutates_args=())
+def append_zero(x: torch.Tensor) -> torch.Tensor:
+    """x [B,T-1,H] with a zero position after the last: the gradient of drop_last."""
+    B, T, H = x.shape[0], x.shape[1] + 1, x.shape[2]
+    return _rows_cut(x, T, 0, torch.empty(B, T, H, dtype=x.dtype, device=x.device))
+
+
+@append_zero.register_fake
+def _(x):
+    return x.new_empty(x.shape[0], x.shape[1] + 1, x.shape[2])
+
+
+drop_last.register_autograd(lambda ctx, g: append_zero(g), setup_context=lambda ctx, inputs, output: None)
+append_zero.register_autograd(lambda ctx, g: drop_last(g), setup_context=lambda ctx, inputs, output: None)
+
+
 @_operator("hawk_b200::linear_ce", mutates_args=())
 def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """(loss [], dweight [V,H] fp32, dact [N,H] fp32) of mean CE(act @ weight^T, labels)."""

@@ -223,6 +223,9 @@ int hawk_decode_norm_linear(const void* residual, const void* pending, const flo
                             void* workspace, size_t workspace_bytes, int B, int H, int N, int res_dtype, int w_dtype,
                             int follows_layer, int* status, void* stream);
 
+/* B sequences of T rows of row_bytes (a multiple of 16): dst [B,T-1] = src [B,T] without each sequence's last row (cut = 1), or
+ * dst [B,T] = src [B,T-1] with a zero row after each sequence (cut = 0). */
+int hawk_rows_cut(const void* src, void* dst, int64_t B, int T, int64_t row_bytes, int cut, void* stream);
 /* The block's forward without gradients, between its large kernels: the fp32 values of conv_w [W,R], conv_b, bx, ba, lam [R]
  * one after the other in out [(W + 4) * R]; and the caches after a prompt: conv_state [B,keep,R] = the last keep rows of the
  * conv's input x [B,T,R] (strides in elements; zero before its first row, hawk/hawk.py:184-190), state [B,R] = the last row of

@@ -262,3 +262,16 @@ def test_core_params_and_cache_store(W, R, T, cache_dtype):
     ops.cache_store(x, h, conv, state)
     want = torch.cat([torch.zeros(3, W - 1, R, device="cuda"), x.float()], 1)[:, T:].to(cache_dtype)
     assert torch.equal(conv, want) and torch.equal(state, h[:, -1:].to(cache_dtype)) and state._version > v
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 2, 8), (3, 2, 64), (5, 129, 72), (2, 513, 2048), (700, 3, 4104)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_drop_last(B, T, H, dt):
+    from hawk_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    x = torch.randn(B, T, H, generator=g, device="cuda").to(dt).requires_grad_()
+    go = torch.randn(B, T - 1, H, generator=g, device="cuda").to(dt)
+    out = ops.drop_last(x)
+    assert out.is_contiguous() and torch.equal(out, x[:, :-1])
+    dx, = torch.autograd.grad(out, x, go)
+    assert torch.equal(dx, torch.nn.functional.pad(go, (0, 0, 0, 1)))
