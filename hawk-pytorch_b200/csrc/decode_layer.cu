@@ -2,6 +2,7 @@
 // head (:300-303), as one chain of seven (two) launches for batches of up to 256 rows:
 //   norm(residual + branch) | input projection | conv + gates + RG-LRU + gelu(y)*h | output projection |
 //   norm(residual + branch) | gate/up projection + gelu(gate)*up | down projection
+// or of five (one) for the fewest, which compute the norms inside the projections.
 //
 // What bounds it: every weight is read once per token, 2.7 GB for the 1.35 B model (0.41 ms at 6.65 TB/s), in launches of
 // 1 to 50 MB each, i.e. 1.3 to 8 us of reading against 2 to 3 us in which a launch drains, the next one starts and its
@@ -27,6 +28,11 @@ using namespace tc;
 // WF32: W is fp32 (a model under autocast) and is rounded to bf16 on its way to shared memory by eight warps, the same
 // rounding that a cast pass makes: 4 bytes of traffic per weight instead of 4 + 2 + 2.
 // GEGLU: W is [gate | up] (2N rows); a tile is 64 gate rows and their 64 up rows and leaves as gelu(gate) * up.
+//
+// Bound by latency and, past 64 tokens, by the partial sums.  16 tokens, back to back over cold weights: 4096 x 2048 7.0 us
+// (8.8 without reading weights early), 2048 x 2048 6.1 (6.8), 2 x 6144 x 2048 with GEGLU 18.7 (20.7), 2048 x 6144 9.6 (10.8),
+// where reading takes 2.5, 1.3, 7.6 and 3.8; of the first, 3.4 us pass between the predecessor's end and the last MMA and 1.8
+// in the cluster's two barriers, the sums and the store.
 // ---------------------------------------------------------------------------------------------
 constexpr int DL_ROWS = 128, DL_BK = 64, DL_W_BYTES = DL_ROWS * DL_BK * 2, DL_MAX_STAGES = 6, DL_MAX_SPLITS = 8;
 // Bytes of a CTA's ring.  Up to 64 tokens three CTAs fit an SM, so that the next launch's are there to read its weights early
@@ -288,7 +294,10 @@ static int linear_launch(const __nv_bfloat16* x, const void* w, int w_dtype, __n
 // time, each its own slice of K, straight from global memory into fragments.  A fragment's k order is free as long as both
 // operands use the same: a lane's 16 bytes (8 consecutive k of one row) serve two MMAs.  The first 16 rows' weights are in
 // registers (64 KB per CTA, two CTAs per SM) before the kernel waits for its predecessor, the next ones are requested
-// before the current ones' sums leave the CTA.  Bound by the weights' bytes for wide layers, by that latency for narrow ones.
+// before the current ones' sums leave the CTA.  Bound by the latency from one launch to the next: of a layer of width 2048, 31 us
+// for one token where its weights take 15.3, 4 each pass between the two norms' inputs and their results, 4 in the recurrent
+// branch's step, 0.6 to 1.7 at each of the five boundaries.  24 layers and the head: 1065 us, 858 with the norm's inputs requested
+// at once, 831 with the branch's step as it is now.
 //
 // NORM: x is the residual (1: bf16, 2: fp32), what is multiplied is norm(x + delta); every CTA computes the statistics of its
 // few rows itself, CTA 0 writes x + delta.  GEGLU: 8 gate rows and their 8 up rows.
