@@ -67,8 +67,24 @@ def lecun_init(w: torch.Tensor, d_in: int) -> None:
     _lecun_normal_(w, d_in)
 
 
+def _fp32_copy(copies: dict, name: str, p: torch.Tensor) -> torch.Tensor:
+    """The fp32 copy of a reduced-precision parameter, kept in `copies` until the parameter is written (version counter) or
+    replaced: by another tensor (`load_state_dict(assign=True)`), which may have the same version, or by other storage
+    (`p.data = t`), which leaves the version as it is.  The entry holds the storage it was made of, so that its address cannot
+    come back with other contents."""
+    if torch.compiler.is_compiling():
+        return p.detach().float()  # a traced graph must not depend on a tensor's version or address
+    hit = copies.get(name)
+    if hit is None or hit[0] is not p or hit[1] != p._version or hit[2].data_ptr() != p.data_ptr() or hit[3].device != p.device:
+        source = p.detach()
+        hit = copies[name] = (p, p._version, source, source.float())
+    return hit[3]
+
+
 class RMSNorm(nn.Module):
     """hawk/hawk.py:47-58: statistics in fp32, result in the input dtype, times the weight."""
+
+    _fp32_cache: Optional[dict] = None
 
     def __init__(self, dim: int, eps: float = 1e-6):
         super().__init__()
@@ -89,11 +105,9 @@ class RMSNorm(nn.Module):
             return w
         if w.requires_grad and torch.is_grad_enabled():
             return w.float()  # training a reduced-precision weight: keep the cast in the autograd graph
-        key = (w.data_ptr(), w._version, w.device)
-        if getattr(self, "_w32_key", None) != key:
-            self._w32 = w.detach().float()
-            self._w32_key = key
-        return self._w32
+        if self._fp32_cache is None:
+            self._fp32_cache = {}
+        return _fp32_copy(self._fp32_cache, "weight", w)
 
     def forward(self, x):
         return ops.rms_norm(x, self._weight32(), self.eps, out_dtype=self._out_dtype(x))
@@ -228,11 +242,7 @@ class Hawk(nn.Module):
         has been cast to bf16 the converted copy is kept until the parameter changes."""
         if p.dtype == torch.float32:
             return p
-        hit = self._fp32_cache.get(name)
-        if hit is None or hit[0] != p._version or hit[1].device != p.device:
-            hit = (p._version, p.detach().float())
-            self._fp32_cache[name] = hit
-        return hit[1]
+        return _fp32_copy(self._fp32_cache, name, p)
 
     def _decode(self, xb_y, cache: RNNCache):
         """One cached token: xb_y [B,1,2R] (hawk/hawk.py:168-179,193-199)."""

@@ -90,3 +90,30 @@ def test_graph_replay_equals_direct_calls():
         dec.prefill(ids[:, :4])
         res.append(torch.cat([dec.step(ids[:, t:t + 1]).clone() for t in range(4, 12)], 1))
     assert torch.equal(res[0], res[1])  # the same kernels in the same order of sums
+
+
+@pytest.mark.parametrize("how", ["assign", "data"])
+def test_cached_token_after_replaced_weights(how):
+    """A bf16 model given other weights decodes as a model built with them (the converted copies of its small parameters
+    follow a replaced parameter, whatever its version)."""
+    torch.manual_seed(5)
+    model, other = (_model(500, 128, 256, 2, 4).bfloat16() for _ in range(2))
+    with torch.no_grad():
+        for p in other.parameters():
+            p.add_(0.05 * torch.randn_like(p))
+    state = {k: v.clone() for k, v in other.state_dict().items()}
+    ids = torch.randint(0, 500, (3, 6), device="cuda")
+
+    def run(m):
+        dec = GraphedDecoder(m, 3, autocast=False, use_graph=False)
+        return [dec.prefill(ids[:, :4]).clone(), dec.step(ids[:, 4:5]).clone()]
+    if how == "assign":  # twice: the parameters of both loads are at version 0
+        model.load_state_dict({k: v.clone() for k, v in model.state_dict().items()}, assign=True)
+    run(model)
+    if how == "assign":
+        model.load_state_dict(state, assign=True)
+    else:
+        for k, p in model.named_parameters():
+            p.data = state[k]
+    for a, b in zip(run(model), run(other)):
+        assert torch.equal(a, b)

@@ -125,3 +125,34 @@ def test_reference_initialiser_names():
     w = torch.empty(512, 256)
     M.lecun_init(w, 256)
     assert abs(float(w.std()) - 1 / math.sqrt(256)) < 0.01 / math.sqrt(256) * 10
+
+
+def _replaced(module, path, value, how):
+    """Fill the parameter `path` of a bf16 module with `value` in one of the ways a program does."""
+    p = module.get_parameter(path)
+    if how == "assign":
+        module.load_state_dict({path: torch.full(p.shape, value, dtype=p.dtype)}, strict=False, assign=True)
+    elif how == "data":
+        p.data = torch.full(p.shape, value, dtype=p.dtype)
+    else:
+        with torch.no_grad():
+            p.fill_(value)
+
+
+@pytest.mark.parametrize("how", ["assign", "data", "write"])
+def test_fp32_copies_follow_the_parameters(how):
+    """The fp32 copies of a bf16 model's small parameters: a replaced parameter can have its predecessor's version, and
+    (freed and allocated again) its predecessor's address."""
+    block = M.Hawk(M.HawkConfig(97, 64, 128, 1, 64, 4, 4)).bfloat16()
+    norm = M.RMSNorm(64).bfloat16()
+    for i in range(1, 9):
+        for name, path in (("w", "conv1d.w"), ("bx", "rg_lru_input_gate.b"), ("lam", "rg_lru_a_param")):
+            _replaced(block, path, float(i), how)
+            if i % 2:  # every other replacement is itself replaced before the copy is asked for
+                _replaced(block, path, float(i) + 0.5, how)
+            got = block._fp32(name, block.get_parameter(path))
+            assert got.dtype == torch.float32 and torch.equal(got, block.get_parameter(path).detach().float()), (i, path)
+        _replaced(norm, "weight", float(i), how)
+        with torch.no_grad():
+            assert torch.equal(norm._weight32(), norm.weight.float())
+    assert block._fp32("lam", block.rg_lru_a_param) is block._fp32("lam", block.rg_lru_a_param)
