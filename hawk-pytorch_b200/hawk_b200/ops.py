@@ -115,9 +115,13 @@ class _on:
 # ---------------------------------------------------------------------------------------------
 # operators
 # ---------------------------------------------------------------------------------------------
+_PLAIN_TYPES = frozenset((type(None), bool, int, float, torch.dtype))
+
+
 def _plain_call(args) -> Optional[bool]:
-    """None where a call belongs to the dispatcher: tracing, transforms, forward-mode derivatives, function and dispatch modes,
-    tensor subclasses, devices other than CUDA.  Otherwise whether autograd has to record it."""
+    """None where a call belongs to the dispatcher: tracing (also by proxies in the place of tensors or numbers), transforms,
+    forward-mode derivatives, function and dispatch modes, tensor subclasses, devices other than CUDA.  Otherwise whether
+    autograd has to record the call."""
     C = torch._C
     if (torch.compiler.is_compiling() or C._len_torch_dispatch_stack() or C._len_torch_function_stack()
             or C._functorch.peek_interpreter_stack() is not None or C._get_tracing_state() is not None
@@ -125,10 +129,13 @@ def _plain_call(args) -> Optional[bool]:
         return None
     grad = False
     for a in args:
-        if isinstance(a, torch.Tensor):
-            if (type(a) is not torch.Tensor and type(a) is not nn.Parameter) or not a.is_cuda:
+        kind = type(a)
+        if kind is torch.Tensor or kind is nn.Parameter:
+            if not a.is_cuda:
                 return None
             grad = grad or a.requires_grad
+        elif kind not in _PLAIN_TYPES:
+            return None
     return grad and torch.is_grad_enabled()
 
 

@@ -1,0 +1,53 @@
+"""Which calls of an operator may run its Python function directly and which belong to torch's dispatcher; on CPU."""
+import pytest
+import torch
+import torch.utils._python_dispatch as python_dispatch
+
+from hawk_b200 import ops
+
+
+class _Passes(torch.overrides.TorchFunctionMode):
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+class _Dispatches(python_dispatch.TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("context", [_Passes, _Dispatches, torch.autograd.forward_ad.dual_level])
+def test_contexts_of_the_dispatcher(context):
+    assert ops._plain_call(()) is False
+    with context():
+        assert ops._plain_call(()) is None
+    assert ops._plain_call(()) is False
+
+
+def test_transforms_and_tracing_belong_to_the_dispatcher():
+    seen = []
+
+    def f(x):
+        seen.append(ops._plain_call(()))
+        return (x * x).sum()
+    torch.func.grad(f)(torch.ones(3))
+    torch.vmap(f)(torch.ones(2, 3))
+    torch.jit.trace(f, torch.ones(3), check_trace=False)
+    assert len(seen) >= 3 and all(s is None for s in seen)
+
+
+def test_arguments_of_the_dispatcher():
+    class Sub(torch.Tensor):
+        pass
+    cpu = torch.ones(2)
+    for args in [(cpu,), (torch.nn.Parameter(cpu),), (cpu.as_subclass(Sub),), (torch.ones(2, device="meta"),), ("text",),
+                 ([cpu],), (torch.fx.Proxy(torch.fx.Graph().placeholder("x")),)]:
+        assert ops._plain_call(args) is None
+    assert ops._plain_call((None, 1, 1.0, True, torch.bfloat16)) is False
+
+
+def test_fx_records_an_operator_as_one_node():
+    def f(x, w, b):
+        return ops.conv1d_fwd(ops.cast_bf16(x), w, b, torch.bfloat16)
+    targets = [str(n.target) for n in torch.fx.symbolic_trace(f).graph.nodes if n.op == "call_function"]
+    assert [t.split(".")[:2] for t in targets] == [["hawk_b200", "cast_bf16"], ["hawk_b200", "conv1d_fwd"]]
