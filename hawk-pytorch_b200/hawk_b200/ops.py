@@ -139,54 +139,68 @@ def _plain_call(args) -> Optional[bool]:
     return grad and torch.is_grad_enabled()
 
 
-class _Operator:
+class _Operator(torch.library.CustomOpDef):
     """A torch.library operator whose ordinary eager calls run its Python function directly, with autograd through one
     torch.autograd.Function.  The dispatcher's way through a Python operator costs 40 to 60 us of host time per call, more
     than most of these kernels take on the GPU: the 24-layer prefill of 3108 tokens (169 such calls) took 12.5 ms against
-    7.8 ms of kernels, a training step of 1551 tokens 7.4 ms against 1.3.  Everything else (see _plain_call) takes it."""
+    7.8 ms of kernels, a training step of 1551 tokens 7.4 ms against 1.3.  Everything else (see _plain_call) takes it, and
+    so does every call once something was registered that the direct way would pass by."""
 
-    def __init__(self, name, mutates_args, fn):
-        self.op = torch.library.custom_op(name, mutates_args=mutates_args)(fn)
-        self.fn, self.function = fn, None
+    @classmethod
+    def make(cls, name, mutates_args, fn):
+        self = torch.library.custom_op(name, mutates_args=mutates_args)(fn)
+        self.__class__ = cls
         names = list(inspect.signature(fn).parameters)
-        self.nargs = len(names)
-        self.mutated = [names.index(m) for m in mutates_args]
+        self.direct, self.direct_fn, self.direct_autograd, self.direct_nargs = True, fn, None, len(names)
+        self.direct_mutated = [names.index(m) for m in mutates_args]
         self.__doc__, self.__name__ = fn.__doc__, fn.__name__
+        return self
 
-    def register_fake(self, fn):
-        return self.op.register_fake(fn)
-
-    def register_autograd(self, backward, *, setup_context):
-        self.op.register_autograd(backward, setup_context=setup_context)
-        fn = self.fn
+    def register_autograd(self, backward, /, *, setup_context=None):
+        super().register_autograd(backward, setup_context=setup_context)
+        fn = self.direct_fn
 
         class Function(torch.autograd.Function):
             @staticmethod
             def forward(ctx, *args):
                 out = fn(*args)
-                setup_context(ctx, args, out)
+                if setup_context is not None:
+                    setup_context(ctx, args, out)
                 return out
 
         Function.backward = staticmethod(backward)
         Function.__name__ = Function.__qualname__ = fn.__name__
-        self.function = Function
+        self.direct_autograd = Function
 
     def __call__(self, *args, **kwargs):
-        if not kwargs and len(args) == self.nargs:
+        if self.direct and not kwargs and len(args) == self.direct_nargs:
             record = _plain_call(args)
             if record is False:
-                out = self.fn(*args)
-                for i in self.mutated:  # what the dispatcher does for a mutated argument
+                out = self.direct_fn(*args)
+                for i in self.direct_mutated:  # what the dispatcher does for a mutated argument
                     if not args[i].is_inference():
                         torch.autograd.graph.increment_version(args[i])
                 return out
-            if record and self.function is not None:
-                return self.function.apply(*args)
-        return self.op(*args, **kwargs)
+            if record and self.direct_autograd is not None:
+                return self.direct_autograd.apply(*args)
+        return super().__call__(*args, **kwargs)
+
+
+def _through_dispatcher(name):
+    def method(self, *args, **kwargs):
+        self.direct = False
+        return getattr(super(_Operator, self), name)(*args, **kwargs)
+    method.__name__ = name
+    return method
+
+
+for _name in ("register_kernel", "register_autocast", "register_torch_dispatch", "register_effect", "set_kernel_enabled"):
+    if hasattr(torch.library.CustomOpDef, _name):
+        setattr(_Operator, _name, _through_dispatcher(_name))
 
 
 def _operator(name, mutates_args):
-    return lambda fn: _Operator(name, mutates_args, fn)
+    return lambda fn: _Operator.make(name, mutates_args, fn)
 
 
 # ---------------------------------------------------------------------------------------------

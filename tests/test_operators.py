@@ -5,6 +5,8 @@ import torch.utils._python_dispatch as python_dispatch
 
 from hawk_b200 import ops
 
+OPERATORS = sorted(k for k, v in vars(ops).items() if isinstance(v, ops._Operator))
+
 
 class _Passes(torch.overrides.TorchFunctionMode):
     def __torch_function__(self, func, types, args=(), kwargs=None):
@@ -51,3 +53,30 @@ def test_fx_records_an_operator_as_one_node():
         return ops.conv1d_fwd(ops.cast_bf16(x), w, b, torch.bfloat16)
     targets = [str(n.target) for n in torch.fx.symbolic_trace(f).graph.nodes if n.op == "call_function"]
     assert [t.split(".")[:2] for t in targets] == [["hawk_b200", "cast_bf16"], ["hawk_b200", "conv1d_fwd"]]
+
+
+def test_operators_are_torch_library_operators():
+    assert len(OPERATORS) >= 34
+    for name in OPERATORS:
+        op = getattr(ops, name)
+        assert isinstance(op, torch.library.CustomOpDef) and op.direct, name
+        assert all(hasattr(op, m) for m in ("register_vmap", "register_kernel", "register_torch_dispatch"))
+
+
+def test_a_registered_kernel_is_used(monkeypatch):
+    @ops._operator("hawk_b200_test::twice", mutates_args=())
+    def twice(x: torch.Tensor) -> torch.Tensor:
+        return 2 * x
+    x = torch.ones(3)
+    monkeypatch.setattr(ops, "_plain_call", lambda args: False)  # as for a plain CUDA tensor
+    assert torch.equal(twice(x), 2 * x)
+    twice.register_kernel("cpu")(lambda x: 3 * x)
+    assert torch.equal(twice(x), 3 * x)
+
+
+def test_a_registered_vmap_rule_is_used():
+    @ops._operator("hawk_b200_test::thrice", mutates_args=())
+    def thrice(x: torch.Tensor) -> torch.Tensor:
+        return 3 * x
+    thrice.register_vmap(lambda info, dims, x: (5 * x, dims[0]))
+    assert torch.equal(torch.vmap(thrice)(torch.ones(2, 3)), torch.full((2, 3), 5.0))
