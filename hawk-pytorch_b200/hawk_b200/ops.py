@@ -115,16 +115,28 @@ class _on:
 # ---------------------------------------------------------------------------------------------
 # operators
 # ---------------------------------------------------------------------------------------------
+def _probes():
+    """What _plain_call asks of torch under private names; None where this torch lacks one of them."""
+    C = torch._C
+    try:
+        torch.autograd.forward_ad._current_level
+        return (C._len_torch_dispatch_stack, C._len_torch_function_stack, C._functorch.peek_interpreter_stack, C._get_tracing_state)
+    except AttributeError:
+        return None
+
+
+_PROBES = _probes()
 _PLAIN_TYPES = frozenset((type(None), bool, int, float, torch.dtype))
 
 
 def _plain_call(args) -> Optional[bool]:
     """None where a call belongs to the dispatcher: tracing (also by proxies in the place of tensors or numbers), transforms,
-    forward-mode derivatives, function and dispatch modes, tensor subclasses, devices other than CUDA.  Otherwise whether
-    autograd has to record the call."""
-    C = torch._C
-    if (torch.compiler.is_compiling() or C._len_torch_dispatch_stack() or C._len_torch_function_stack()
-            or C._functorch.peek_interpreter_stack() is not None or C._get_tracing_state() is not None
+    forward-mode derivatives, function and dispatch modes, tensor subclasses, devices other than CUDA; and always where torch
+    cannot be asked.  Otherwise whether autograd has to record the call."""
+    if torch.compiler.is_compiling() or _PROBES is None:
+        return None
+    dispatch_modes, function_modes, transform, tracing = _PROBES
+    if (dispatch_modes() or function_modes() or transform() is not None or tracing() is not None
             or torch.autograd.forward_ad._current_level >= 0):
         return None
     grad = False

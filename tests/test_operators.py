@@ -48,6 +48,13 @@ def test_arguments_of_the_dispatcher():
     assert ops._plain_call((None, 1, 1.0, True, torch.bfloat16)) is False
 
 
+def test_a_torch_without_the_private_names_takes_the_dispatcher(monkeypatch):
+    monkeypatch.delattr(torch._C, "_len_torch_function_stack")
+    assert ops._probes() is None
+    monkeypatch.setattr(ops, "_PROBES", None)
+    assert ops._plain_call(()) is None
+
+
 def test_fx_records_an_operator_as_one_node():
     def f(x, w, b):
         return ops.conv1d_fwd(ops.cast_bf16(x), w, b, torch.bfloat16)
