@@ -119,7 +119,7 @@ def _probes():
     """What _plain_call asks of torch under private names; None where this torch lacks one of them."""
     C = torch._C
     try:
-        torch.autograd.forward_ad._current_level
+        torch.autograd.forward_ad._current_level, torch.autograd.profiler._is_profiler_enabled
         return (C._len_torch_dispatch_stack, C._len_torch_function_stack, C._functorch.peek_interpreter_stack, C._get_tracing_state)
     except AttributeError:
         return None
@@ -131,13 +131,14 @@ _PLAIN_TYPES = frozenset((type(None), bool, int, float, torch.dtype))
 
 def _plain_call(args) -> Optional[bool]:
     """None where a call belongs to the dispatcher: tracing (also by proxies in the place of tensors or numbers), transforms,
-    forward-mode derivatives, function and dispatch modes, tensor subclasses, devices other than CUDA; and always where torch
-    cannot be asked.  Otherwise whether autograd has to record the call."""
+    forward-mode derivatives, function and dispatch modes, a running profiler (which knows operators by the dispatcher),
+    tensor subclasses, devices other than CUDA; and always where torch cannot be asked.  Otherwise whether autograd has to
+    record the call."""
     if torch.compiler.is_compiling() or _PROBES is None:
         return None
     dispatch_modes, function_modes, transform, tracing = _PROBES
     if (dispatch_modes() or function_modes() or transform() is not None or tracing() is not None
-            or torch.autograd.forward_ad._current_level >= 0):
+            or torch.autograd.forward_ad._current_level >= 0 or torch.autograd.profiler._is_profiler_enabled):
         return None
     grad = False
     for a in args:

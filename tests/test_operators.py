@@ -18,7 +18,8 @@ class _Dispatches(python_dispatch.TorchDispatchMode):
         return func(*args, **(kwargs or {}))
 
 
-@pytest.mark.parametrize("context", [_Passes, _Dispatches, torch.autograd.forward_ad.dual_level])
+@pytest.mark.parametrize("context", [_Passes, _Dispatches, torch.autograd.forward_ad.dual_level, torch.profiler.profile,
+                                     torch.autograd.profiler.profile])
 def test_contexts_of_the_dispatcher(context):
     assert ops._plain_call(()) is False
     with context():
