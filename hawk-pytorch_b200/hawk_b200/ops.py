@@ -919,7 +919,9 @@ def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
     lib = _lib.load()
     V, H = weight.shape
     N = act.shape[0]
-    weight, act, labels = weight.contiguous(), act.contiguous(), labels.contiguous()
+    weight, labels = weight.contiguous(), labels.contiguous()
+    # operands of two types: act may lie at any address (a cast to the weight's type would have moved it)
+    act = act.contiguous() if act.dtype == weight.dtype else _dense16(act)
     if labels.dtype != torch.int64:
         labels = labels.long()
     loss = torch.empty((), dtype=torch.float32, device=act.device)
@@ -951,7 +953,8 @@ def linear_ce_bwd(weight: torch.Tensor, act: torch.Tensor, saved: torch.Tensor, 
     lib = _lib.load()
     V, H = weight.shape
     N = act.shape[0]
-    weight, act = weight.contiguous(), act.contiguous()
+    weight = weight.contiguous()
+    act = act.contiguous() if act.dtype == weight.dtype else _dense16(act)
     g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
     dw = torch.empty((V, H) if want_dw else 0, dtype=weight.dtype, device=act.device)
     da = torch.empty((N, H) if want_da else 0, dtype=act.dtype, device=act.device)
@@ -992,8 +995,10 @@ def fused_cross_entropy(lm_head_weight, act, labels):
     """Mean cross-entropy of `act @ lm_head_weight.T` against `labels`; drop-in for
     hawk/fused_cross_entropy.py:77-79.  weight [V,H], act [N,H] (fp32 or bf16), labels [N] int64.
     The arithmetic is the reference's under bf16 autocast whether or not autocast is on: bf16
-    tensor-core GEMMs with fp32 accumulation, bf16 logits, fp32 softmax.  weight and act may differ in dtype; each
-    gradient has its operand's."""
+    tensor-core GEMMs with fp32 accumulation, bf16 logits, fp32 softmax.  weight and act may differ in dtype (an act
+    that is neither fp32 nor bf16 is converted to the weight's); each gradient has its operand's."""
+    if act.dtype not in (torch.float32, torch.bfloat16):
+        act = act.to(lm_head_weight.dtype)
     want_grad = torch.is_grad_enabled() and (lm_head_weight.requires_grad or act.requires_grad)
     return linear_ce_fwd(lm_head_weight, act, labels, want_grad)[0]
 

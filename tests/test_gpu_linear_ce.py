@@ -167,3 +167,35 @@ def test_linear_ce_tiles_and_splits(N, H, V, wdt, adt):
     (1.7 * ref).backward()
     assert wd.grad.dtype == wdt and ad.grad.dtype == adt and abs(float(loss) - float(ref)) <= TOL * float(ref)
     assert rel_l2(wd.grad, w64.grad) <= TOL and rel_l2(ad.grad, a64.grad) <= TOL
+
+
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("adt", [torch.float16, torch.float64])
+def test_act_of_other_types_is_converted_to_the_weights(wdt, adt):
+    from hawk_b200 import fused_cross_entropy
+    w, act, labels = _case(200, 64, 300, seed=1)
+    w, labels = w.to("cuda", wdt).requires_grad_(), labels.cuda()
+    other = act.to("cuda", adt).requires_grad_()
+    same = other.detach().to(wdt).requires_grad_()
+    losses = [fused_cross_entropy(w, a, labels) for a in (other, same)]
+    grads = [torch.autograd.grad(1.7 * loss, (w, a)) for loss, a in zip(losses, (other, same))]
+    assert torch.equal(losses[0], losses[1]) and torch.equal(grads[0][0], grads[1][0])
+    assert grads[0][1].dtype == adt and torch.equal(grads[0][1], grads[1][1].to(adt))
+
+
+@pytest.mark.parametrize("wdt,adt", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+def test_act_of_the_other_type_at_any_address(wdt, adt):
+    from hawk_b200 import fused_cross_entropy
+    N, H = 200, 64
+    w, act, labels = _case(N, H, 300, seed=2)
+    w, labels = w.to("cuda", wdt).requires_grad_(), labels.cuda()
+    flat = torch.empty(1 + N * H, dtype=adt, device="cuda")
+    flat[1:] = act.to("cuda", adt).view(-1)
+    odd = flat[1:].view(N, H).requires_grad_()
+    even = odd.detach().clone().requires_grad_()
+    assert odd.data_ptr() % 16 and not even.data_ptr() % 16
+    res = []
+    for a in (odd, even):
+        loss = fused_cross_entropy(w, a, labels)
+        res.append([loss, *torch.autograd.grad(1.7 * loss, (w, a))])
+    assert all(torch.equal(p, q) for p, q in zip(*res))
