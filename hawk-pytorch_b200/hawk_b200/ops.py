@@ -890,9 +890,9 @@ def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor) -> 
     loss = torch.empty((), dtype=torch.float32, device=act.device)
     dweight = torch.empty(V, H, dtype=torch.float32, device=act.device)
     dact = torch.empty(N, H, dtype=torch.float32, device=act.device)
-    ws_bytes = lib.hawk_linear_ce_workspace_bytes(N, H, V)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=act.device)
     with _on(act, "linear_ce", 10 if weight.dtype == torch.float32 else 8):
+        ws_bytes = lib.hawk_linear_ce_workspace_bytes(N, H, V)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=act.device)
         _lib.check(lib.hawk_linear_ce_fwd_bwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(),
                                               dweight.data_ptr(), dact.data_ptr(), ws.data_ptr(), ws_bytes, N, H, V,
                                               _dt(weight), _status_word(act.device).data_ptr(), _stream(act)),
@@ -926,9 +926,10 @@ def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
         labels = labels.long()
     loss = torch.empty((), dtype=torch.float32, device=act.device)
     saved = torch.empty(lib.hawk_linear_ce_saved_bytes(N, H, V, _dt(weight), _dt(act)), dtype=torch.uint8, device=act.device)
-    ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
     casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
     with _on(act, "linear_ce", 3 + casts + bool(want_grad)):
+        # asked on the operands' device: the K splits, and with them the size, follow its SM count
+        ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
         _lib.check(lib.hawk_linear_ce_fwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(),
                                           saved.data_ptr(), saved.numel(), ws.data_ptr(), ws.numel(), N, H, V, _dt(weight),
                                           _dt(act), int(want_grad), _status_word(act.device).data_ptr(), _stream(act)),
@@ -958,8 +959,8 @@ def linear_ce_bwd(weight: torch.Tensor, act: torch.Tensor, saved: torch.Tensor, 
     g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
     dw = torch.empty((V, H) if want_dw else 0, dtype=weight.dtype, device=act.device)
     da = torch.empty((N, H) if want_da else 0, dtype=act.dtype, device=act.device)
-    ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
     with _on(act, "linear_ce", 1 + want_dw + want_da):
+        ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
         _lib.check(lib.hawk_linear_ce_bwd(weight.data_ptr(), act.data_ptr(), saved.data_ptr(), saved.numel(), g.data_ptr(),
                                           dw.data_ptr() if want_dw else None, _dt(weight),
                                           da.data_ptr() if want_da else None, _dt(act), ws.data_ptr(), ws.numel(), N, H, V,

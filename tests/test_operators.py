@@ -88,3 +88,33 @@ def test_a_registered_vmap_rule_is_used():
         return 3 * x
     thrice.register_vmap(lambda info, dims, x: (5 * x, dims[0]))
     assert torch.equal(torch.vmap(thrice)(torch.ones(2, 3)), torch.full((2, 3), 5.0))
+
+
+def test_linear_ce_sizes_are_asked_on_the_operands_device(monkeypatch):
+    """The K splits of the gradient GEMMs follow the current device's SM count, so the calls that size their scratch belong
+    under the same device guard as the calls that use it."""
+    inside = []
+
+    class Guard:
+        def __init__(self, *args):
+            pass
+
+        def __enter__(self):
+            inside.append(1)
+
+        def __exit__(self, *exc):
+            inside.pop()
+
+    class Lib:
+        def __getattr__(self, name):
+            def call(*args):
+                assert inside or name == "hawk_linear_ce_saved_bytes", name
+                return 256 if name.endswith("_bytes") else 0
+            return call
+    monkeypatch.setattr(ops._lib, "load", Lib)
+    monkeypatch.setattr(ops, "_on", Guard)
+    monkeypatch.setattr(ops, "_stream", lambda t: 0)
+    monkeypatch.setattr(ops, "_status_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    w, act, labels = torch.ones(4, 8, requires_grad=True), torch.ones(3, 8, requires_grad=True), torch.zeros(3, dtype=torch.long)
+    torch.autograd.grad(ops.fused_cross_entropy(w, act, labels), (w, act))
+    ops.linear_ce(w.detach(), act.detach(), labels)
