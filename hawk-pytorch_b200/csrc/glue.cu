@@ -131,6 +131,25 @@ __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restr
   }
 }
 
+// dst = src * *scale in dst's type: a gradient that was formed before the loss's own gradient was known.  One pass of 16-byte
+// accesses (torch's multiplication by a 0-dimensional tensor: 171 us for 32760 x 2048 to fp32, 230 to bf16 in two passes,
+// where 82 and 62 us of traffic at the copy rate move; this kernel 84 and 66).
+template <typename TO>
+__global__ void __launch_bounds__(256)
+scale_kernel(const float* __restrict__ src, const float* __restrict__ scale, TO* __restrict__ dst, int64_t n) {
+  const float g = *scale;
+  const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
+  if (i + 8 <= n) {
+    float v[8];
+    VecIO<float, 8>::load(src + i, v);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] *= g;
+    VecIO<TO, 8>::store(dst + i, v);
+  } else {
+    for (int64_t j = i; j < n; ++j) dst[j] = from_float<TO>(src[j] * g);
+  }
+}
+
 // Rows of nv 16-byte words, in sequences of T: dst = src without each sequence's last row (cut), or src with a zero row after
 // each sequence (the cut's gradient).  The next-token loss cuts the last position off: torch's strided copy of 8 x 4096 x 2048
 // bf16 took 199 us either way, plus a fill, where 268 MB move (40 us).
@@ -523,6 +542,18 @@ extern "C" int hawk_cast_f32_bf16(const float* src, void* dst, int64_t n, void* 
   HAWK_REQUIRE(aligned(src, 16) && aligned(dst, 16), HAWK_ERR_ALIGN);
   cast_f32_bf16_kernel<<<grid_for(n / 8 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       src, static_cast<bf*>(dst), n);
+  return launch_status();
+}
+
+extern "C" int hawk_scale(const float* src, const float* scale, void* dst, int64_t n, int dst_dtype, void* stream) {
+  HAWK_REQUIRE(src && scale && dst, HAWK_ERR_NULL);
+  HAWK_REQUIRE(valid_dtype(dst_dtype), HAWK_ERR_DTYPE);
+  HAWK_REQUIRE(n >= 1 && n <= (1LL << 40), HAWK_ERR_SHAPE);
+  HAWK_REQUIRE(aligned(src, 16) && aligned(dst, 16) && aligned(scale, 4), HAWK_ERR_ALIGN);
+  const unsigned blocks = (unsigned)((n + 2047) / 2048);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dst_dtype == HAWK_BF16) scale_kernel<<<blocks, 256, 0, st>>>(src, scale, static_cast<bf*>(dst), n);
+  else scale_kernel<<<blocks, 256, 0, st>>>(src, scale, static_cast<float*>(dst), n);
   return launch_status();
 }
 

@@ -1,8 +1,8 @@
-// Fused linear + cross-entropy: the loss in the forward call, d act and d weight in the backward call, replacing
+// Fused linear + cross-entropy: the loss in one call, d act and d weight in a second, replacing
 // hawk/fused_cross_entropy.py:11-73 (2048-row chunks, three cuBLAS GEMMs and ~8 passes over
 // [chunk, V] fp32 temporaries per chunk).
 //
-// Forward, all on the caller's stream:
+// Loss, all on the caller's stream:
 //   1. cast           : fp32 weight [V,H] and act [N,H] -> bf16 copies (bf16 inputs are used in place).
 //   2. GEMM + softmax epilogue (tcgen05): logits tile = act @ weight^T accumulated in TMEM; the
 //      epilogue rounds it to bf16 (as F.linear does under autocast, fused_cross_entropy.py:28),
@@ -11,11 +11,11 @@
 //   3. row reduce     : tile statistics -> log-sum-exp per row, loss = mean(lse - correct) (:37-44,59-64).
 //   4. dprobs         : logits -> (softmax - onehot) / N in bf16, in place (:47-52); skipped when no gradient
 //                       is wanted.
-// Backward: two GEMMs with a plain epilogue that multiplies by the incoming gradient of the loss,
+// Gradients: two GEMMs with a plain epilogue that can multiply by a gradient of the loss,
 //      d act = dprobs @ weight (:56), d weight = dprobs^T @ act (:55).  Neither needs a transposed copy: an operand
 //      whose contraction index is the row index of its tensor (weight in d act; dprobs and act in d weight) is read
-//      as an MN-major tile straight from the row-major tensor.  The forward leaves dprobs and the bf16 operands
-//      behind for it, so no pass over [V,H] or [N,H] fp32 gradients follows the GEMMs.
+//      as an MN-major tile straight from the row-major tensor.  The first call leaves dprobs and the bf16 operands
+//      behind for it.
 //
 // The GEMM is one kernel: C[M,Nc] = A[M,K] . B[Nc,K]^T, bf16 operands, fp32 accumulation.
 // A pair of CTAs (cta_group::2) computes a 256*MH x 256 output tile, K in blocks of 64 (128-byte swizzled rows).  What

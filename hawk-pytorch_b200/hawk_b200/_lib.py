@@ -14,7 +14,7 @@ LIB_PATH = os.path.join(_HERE, "libhawk_b200.so")
 
 HAWK_F32 = 0
 HAWK_BF16 = 1
-ABI_VERSION = 5
+ABI_VERSION = 6
 
 _P = c_void_p
 
@@ -59,6 +59,7 @@ SIGNATURES = {
     "hawk_decode_norm_linear": (c_int, [_P, _P, _P, c_float, _P, _P, _P, c_size_t] + [c_int] * 6 + [_P, _P]),
     "hawk_adamw_step": (c_int, [_P, _P, _P, _P, _P, c_int64, c_float, c_float, c_float, c_float, c_float, c_int64, _P]),
     "hawk_adamw_multi": (c_int, [c_char_p, c_int, c_float, c_float, c_float, c_float, c_float, c_int64, _P]),
+    "hawk_scale": (c_int, [_P, _P, _P, c_int64, c_int, _P]),
     "hawk_cast_f32_bf16": (c_int, [_P, _P, c_int64, _P]),
     "hawk_gelu_mul_fwd": (c_int, [_P, c_int64, _P, c_int64, _P, c_int64, c_int64, c_int, c_int, _P]),
     "hawk_gelu_mul_bwd": (c_int, [_P, c_int64, _P, c_int64, _P, c_int64, _P, c_int64, _P, c_int64, c_int64, c_int,

@@ -878,63 +878,114 @@ drop_last.register_autograd(lambda ctx, g: append_zero(g), setup_context=lambda 
 append_zero.register_autograd(lambda ctx, g: drop_last(g), setup_context=lambda ctx, inputs, output: None)
 
 
-@_operator("hawk_b200::linear_ce", mutates_args=())
-def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """(loss [], dweight [V,H] fp32, dact [N,H] fp32) of mean CE(act @ weight^T, labels)."""
+def _ce_forward(weight, act, labels, want_grad):
+    """(loss, saved): `saved` holds d logits and the bf16 copies of fp32 operands (want_grad), else what the call leaves."""
     lib = _lib.load()
     V, H = weight.shape
     N = act.shape[0]
-    weight, act, labels = weight.contiguous(), act.contiguous(), labels.contiguous()
-    if labels.dtype != torch.int64:
-        labels = labels.long()
-    loss = torch.empty((), dtype=torch.float32, device=act.device)
-    dweight = torch.empty(V, H, dtype=torch.float32, device=act.device)
-    dact = torch.empty(N, H, dtype=torch.float32, device=act.device)
-    with _on(act, "linear_ce", 10 if weight.dtype == torch.float32 else 8):
-        ws_bytes = lib.hawk_linear_ce_workspace_bytes(N, H, V)
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=act.device)
-        _lib.check(lib.hawk_linear_ce_fwd_bwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(),
-                                              dweight.data_ptr(), dact.data_ptr(), ws.data_ptr(), ws_bytes, N, H, V,
-                                              _dt(weight), _status_word(act.device).data_ptr(), _stream(act)),
-                   "hawk_linear_ce_fwd_bwd")
-    return loss, dweight, dact
-
-
-@linear_ce.register_fake
-def _(weight, act, labels):
-    return (act.new_empty((), dtype=torch.float32), weight.new_empty(weight.shape, dtype=torch.float32),
-            act.new_empty(act.shape, dtype=torch.float32))
-
-
-linear_ce.register_autograd(
-    lambda ctx, g_loss, g_dw, g_da: tuple((g_loss * t).to(dt) for t, dt in zip(ctx.saved_tensors, ctx.dtypes)) + (None,),
-    setup_context=lambda ctx, inputs, output: (ctx.save_for_backward(*output[1:]),
-                                               setattr(ctx, "dtypes", (inputs[0].dtype, inputs[1].dtype)))[0])
-
-
-@_operator("hawk_b200::linear_ce_fwd", mutates_args=())
-def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
-                  want_grad: bool) -> Tuple[torch.Tensor, torch.Tensor]:
-    """(loss [], saved): mean CE(act @ weight^T, labels) and, with want_grad, what linear_ce_bwd needs."""
-    lib = _lib.load()
-    V, H = weight.shape
-    N = act.shape[0]
-    weight, labels = weight.contiguous(), labels.contiguous()
-    # operands of two types: act may lie at any address (a cast to the weight's type would have moved it)
-    act = act.contiguous() if act.dtype == weight.dtype else _dense16(act)
     if labels.dtype != torch.int64:
         labels = labels.long()
     loss = torch.empty((), dtype=torch.float32, device=act.device)
     saved = torch.empty(lib.hawk_linear_ce_saved_bytes(N, H, V, _dt(weight), _dt(act)), dtype=torch.uint8, device=act.device)
-    casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
-    with _on(act, "linear_ce", 3 + casts + bool(want_grad)):
-        # asked on the operands' device: the K splits, and with them the size, follow its SM count
-        ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
-        _lib.check(lib.hawk_linear_ce_fwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(),
-                                          saved.data_ptr(), saved.numel(), ws.data_ptr(), ws.numel(), N, H, V, _dt(weight),
-                                          _dt(act), int(want_grad), _status_word(act.device).data_ptr(), _stream(act)),
-                   "hawk_linear_ce_fwd")
+    ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
+    _lib.check(lib.hawk_linear_ce_fwd(weight.data_ptr(), act.data_ptr(), labels.data_ptr(), loss.data_ptr(), saved.data_ptr(),
+                                      saved.numel(), ws.data_ptr(), ws.numel(), N, H, V, _dt(weight), _dt(act), int(want_grad),
+                                      _status_word(act.device).data_ptr(), _stream(act)), "hawk_linear_ce_fwd")
     return loss, saved
+
+
+def _ce_grads(weight, act, saved, grad_loss, dw, da):
+    """dw [V,H] and da [N,H] (None: not wanted) filled from what _ce_forward left, times grad_loss (None: 1)."""
+    lib = _lib.load()
+    V, H = weight.shape
+    N = act.shape[0]
+    ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
+    _lib.check(lib.hawk_linear_ce_bwd(weight.data_ptr(), act.data_ptr(), saved.data_ptr(), saved.numel(), _ptr(grad_loss),
+                                      _ptr(dw), _dt(weight if dw is None else dw), _ptr(da), _dt(act if da is None else da),
+                                      ws.data_ptr(), ws.numel(), N, H, V, _dt(weight), _dt(act),
+                                      _status_word(act.device).data_ptr(), _stream(act)), "hawk_linear_ce_bwd")
+
+
+def _ce_operands(weight, act, labels=None):
+    # operands of two types: act may lie at any address (a cast to the weight's type would have moved it)
+    act = act.contiguous() if act.dtype == weight.dtype else _dense16(act)
+    return weight.contiguous(), act, None if labels is None else labels.contiguous()
+
+
+@_operator("hawk_b200::linear_ce", mutates_args=())
+def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor, want_dw: bool = True,
+              want_da: bool = True) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """(loss [], dweight [V,H] fp32, dact [N,H] fp32) of mean CE(act @ weight^T, labels); a gradient that is not wanted is
+    empty.  Formed in the forward call, as in the reference (hawk/fused_cross_entropy.py:52-63): a loss that waits for its
+    backward holds these and not [N,V] probabilities, and its operands may be written meanwhile.  What that costs is the
+    backward's pass over them: N32760 H2048 V32000 11.46 ms, 11.42 with the gradients formed in the backward call."""
+    weight, act, labels = _ce_operands(weight, act, labels)
+    (V, H), N = weight.shape, act.shape[0]
+    casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
+    want = want_dw or want_da
+    with _on(act, "linear_ce", 3 + casts + (2 + want_dw + want_da if want else 0)):
+        loss, saved = _ce_forward(weight, act, labels, want)
+        dw = torch.empty((V, H) if want_dw else 0, dtype=torch.float32, device=act.device)
+        da = torch.empty((N, H) if want_da else 0, dtype=torch.float32, device=act.device)
+        if want:
+            _ce_grads(weight, act, saved, None, dw if want_dw else None, da if want_da else None)
+    return loss, dw, da
+
+
+@linear_ce.register_fake
+def _(weight, act, labels, want_dw=True, want_da=True):
+    return (act.new_empty((), dtype=torch.float32), weight.new_empty(weight.shape if want_dw else 0, dtype=torch.float32),
+            act.new_empty(act.shape if want_da else 0, dtype=torch.float32))
+
+
+@_operator("hawk_b200::scaled", mutates_args=())
+def scaled(x: torch.Tensor, scale: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """x (fp32) times the scalar `scale`, in `dtype`."""
+    lib = _lib.load()
+    x, scale = _dense16(x), scale.float()
+    out = torch.empty(x.shape, dtype=dtype, device=x.device)
+    if x.numel():
+        with _on(x, "scaled", 1):
+            _lib.check(lib.hawk_scale(x.data_ptr(), scale.data_ptr(), out.data_ptr(), x.numel(), _dt(out), _stream(x)), "hawk_scale")
+    return out
+
+
+@scaled.register_fake
+def _(x, scale, dtype):
+    return x.new_empty(x.shape, dtype=dtype)
+
+
+def _ce_setup(ctx, inputs, output):
+    weight, act, _, ctx.want_dw, ctx.want_da = inputs
+    ctx.save_for_backward(*output[1:])
+    ctx.dtypes = (weight.dtype, act.dtype)
+    ctx.set_materialize_grads(False)
+
+
+def _ce_backward(ctx, g_loss, g_dw, g_da):
+    if g_loss is None:
+        return None, None, None, None, None
+    if torch.is_grad_enabled():  # create_graph: an expression that can be differentiated
+        times = lambda t, dt: (g_loss * t).to(dt)  # noqa: E731
+    else:
+        times = lambda t, dt: scaled(t, g_loss, dt)  # noqa: E731
+    dw, da = (times(t, dt) if want else None
+              for t, dt, want in zip(ctx.saved_tensors, ctx.dtypes, (ctx.want_dw, ctx.want_da)))
+    return dw, da, None, None, None
+
+
+linear_ce.register_autograd(_ce_backward, setup_context=_ce_setup)
+
+
+# the two calls of linear_ce by themselves
+@_operator("hawk_b200::linear_ce_fwd", mutates_args=())
+def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
+                  want_grad: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(loss [], saved): mean CE(act @ weight^T, labels) and, with want_grad, what linear_ce_bwd needs."""
+    weight, act, labels = _ce_operands(weight, act, labels)
+    casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
+    with _on(act, "linear_ce_fwd", 3 + casts + bool(want_grad)):
+        return _ce_forward(weight, act, labels, want_grad)
 
 
 @linear_ce_fwd.register_fake
@@ -951,45 +1002,18 @@ def _(weight, act, labels, want_grad):
 def linear_ce_bwd(weight: torch.Tensor, act: torch.Tensor, saved: torch.Tensor, grad_loss: torch.Tensor, want_dw: bool,
                   want_da: bool) -> Tuple[torch.Tensor, torch.Tensor]:
     """(d weight, d act) in the operands' dtypes, times grad_loss (empty where not wanted)."""
-    lib = _lib.load()
-    V, H = weight.shape
-    N = act.shape[0]
-    weight = weight.contiguous()
-    act = act.contiguous() if act.dtype == weight.dtype else _dense16(act)
+    weight, act, _ = _ce_operands(weight, act)
     g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
-    dw = torch.empty((V, H) if want_dw else 0, dtype=weight.dtype, device=act.device)
-    da = torch.empty((N, H) if want_da else 0, dtype=act.dtype, device=act.device)
-    with _on(act, "linear_ce", 1 + want_dw + want_da):
-        ws = torch.empty(lib.hawk_linear_ce_scratch_bytes(N, H, V), dtype=torch.uint8, device=act.device)
-        _lib.check(lib.hawk_linear_ce_bwd(weight.data_ptr(), act.data_ptr(), saved.data_ptr(), saved.numel(), g.data_ptr(),
-                                          dw.data_ptr() if want_dw else None, _dt(weight),
-                                          da.data_ptr() if want_da else None, _dt(act), ws.data_ptr(), ws.numel(), N, H, V,
-                                          _dt(weight), _dt(act), _status_word(act.device).data_ptr(), _stream(act)),
-                   "hawk_linear_ce_bwd")
+    dw = torch.empty(weight.shape if want_dw else 0, dtype=weight.dtype, device=act.device)
+    da = torch.empty(act.shape if want_da else 0, dtype=act.dtype, device=act.device)
+    with _on(act, "linear_ce_bwd", 1 + want_dw + want_da):
+        _ce_grads(weight, act, saved, g, dw if want_dw else None, da if want_da else None)
     return dw, da
 
 
 @linear_ce_bwd.register_fake
 def _(weight, act, saved, grad_loss, want_dw, want_da):
     return (weight.new_empty(weight.shape if want_dw else 0), act.new_empty(act.shape if want_da else 0))
-
-
-def _ce_setup(ctx, inputs, output):
-    weight, act, _, want_grad = inputs
-    assert want_grad, "linear_ce_fwd(want_grad=False) cannot be differentiated"
-    ctx.save_for_backward(weight, act, output[1])
-    ctx.set_materialize_grads(False)
-
-
-def _ce_backward(ctx, g_loss, g_saved):
-    if g_loss is None:
-        return None, None, None, None
-    want_dw, want_da = ctx.needs_input_grad[:2]
-    dw, da = linear_ce_bwd(*ctx.saved_tensors, g_loss, want_dw, want_da)
-    return dw if want_dw else None, da if want_da else None, None, None
-
-
-linear_ce_fwd.register_autograd(_ce_backward, setup_context=_ce_setup)
 
 
 def fused_cross_entropy(lm_head_weight, act, labels):
@@ -1000,8 +1024,8 @@ def fused_cross_entropy(lm_head_weight, act, labels):
     that is neither fp32 nor bf16 is converted to the weight's); each gradient has its operand's."""
     if act.dtype not in (torch.float32, torch.bfloat16):
         act = act.to(lm_head_weight.dtype)
-    want_grad = torch.is_grad_enabled() and (lm_head_weight.requires_grad or act.requires_grad)
-    return linear_ce_fwd(lm_head_weight, act, labels, want_grad)[0]
+    grad = torch.is_grad_enabled()
+    return linear_ce(lm_head_weight, act, labels, grad and lm_head_weight.requires_grad, grad and act.requires_grad)[0]
 
 
 class CrossEntropyLoopedFused:

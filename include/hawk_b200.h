@@ -28,7 +28,7 @@
 extern "C" {
 #endif
 
-#define HAWK_B200_ABI_VERSION 5
+#define HAWK_B200_ABI_VERSION 6
 
 typedef enum hawk_dtype { HAWK_F32 = 0, HAWK_BF16 = 1 } hawk_dtype;
 
@@ -255,7 +255,7 @@ int hawk_cache_store(const void* x, int64_t x_batch_stride, int64_t x_row_stride
  * it has no ignore_index): a label outside the range makes `loss` non-finite (NaN or inf).
  * ---------------------------------------------------------------------------------------- */
 size_t hawk_linear_ce_workspace_bytes(int64_t N, int64_t H, int64_t V);
-/* The same computation as two calls, as autograd runs it.  hawk_linear_ce_fwd writes the loss and, with want_grad,
+/* The same computation as two calls, each gradient on demand.  hawk_linear_ce_fwd writes the loss and, with want_grad,
  * leaves dprobs and the bf16 copies of fp32 operands in `saved` (hawk_linear_ce_saved_bytes, 256-byte aligned);
  * hawk_linear_ce_bwd turns them into dweight [V,H] and dact [N,H] (either may be NULL), in fp32 or bf16, times the
  * device scalar *grad_loss (NULL: 1).  weight and act are the forward's, in w_dtype / a_dtype (they may differ), and are
@@ -349,6 +349,8 @@ int hawk_add_rms_norm_bwd(const void* dy, const void* x_sum, const float* w, con
  * before every bf16 GEMM of an fp32 parameter (torch's type-converting copy, reached from F.linear in
  * hawk/hawk.py:75-86,110-116 under torch.autocast), as one vectorised pass.  src, dst 16-byte aligned. */
 int hawk_cast_f32_bf16(const float* src, void* dst, int64_t n, void* stream);
+/* dst[n] = src[n] * *scale (a device scalar) in dst_dtype: the backward of hawk_linear_ce_fwd_bwd's gradients; 16-byte aligned. */
+int hawk_scale(const float* src, const float* scale, void* dst, int64_t n, int dst_dtype, void* stream);
 
 /* One AdamW step (decoupled weight decay, torch.optim.AdamW's update rule with bias correction for
  * step number `step` >= 1) on n contiguous fp32 elements, in place in p, m (first moment) and v (second

@@ -199,3 +199,47 @@ def test_act_of_the_other_type_at_any_address(wdt, adt):
         loss = fused_cross_entropy(w, a, labels)
         res.append([loss, *torch.autograd.grad(1.7 * loss, (w, a))])
     assert all(torch.equal(p, q) for p, q in zip(*res))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_loss_waiting_for_its_backward(dtype):
+    """Between the loss and backward(): the operands may be written, and what is held is no larger than the fp32 gradients
+    (an [N,V] tensor would be 2 N V = 15 MB here, the gradients are 2.6 MB)."""
+    from hawk_b200 import fused_cross_entropy
+    N, H, V = 2500, 64, 3000
+    w, act, labels = _case(N, H, V, seed=3)
+    w, act, labels = w.to("cuda", dtype).requires_grad_(), act.to("cuda", dtype).requires_grad_(), labels.cuda()
+    want = torch.autograd.grad(1.7 * fused_cross_entropy(w, act, labels), (w, act))
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    loss = fused_cross_entropy(w, act, labels)
+    held = torch.cuda.memory_allocated() - before
+    assert held <= 4 * H * (N + V) + 4096, held
+    with torch.no_grad():
+        w.zero_()
+        act.mul_(3)
+    twice = [torch.autograd.grad(1.7 * loss, (w, act), retain_graph=keep) for keep in (True, False)]
+    assert all(torch.equal(a, b) for got in twice for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_gradient_of_one_operand_only(which):
+    from hawk_b200 import fused_cross_entropy
+    w, act, labels = _case(300, 64, 500, seed=4)
+    both = [w.cuda().requires_grad_(), act.cuda().requires_grad_()]
+    want = torch.autograd.grad(fused_cross_entropy(*both, labels.cuda()), both)[which]
+    one = [t.detach().requires_grad_(i == which) for i, t in enumerate(both)]
+    fused_cross_entropy(*one, labels.cuda()).backward()
+    assert torch.equal(one[which].grad, want) and one[1 - which].grad is None
+    with torch.no_grad():
+        assert not fused_cross_entropy(*both, labels.cuda()).requires_grad
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 2047, 2048, 5001])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_scaled(n, dtype):
+    from hawk_b200 import ops
+    flat = torch.randn(n + 1, device="cuda")
+    g = torch.tensor(1.7, device="cuda")
+    for x in (flat[:n], flat[1:]):  # at an aligned and an odd address
+        assert torch.equal(ops.scaled(x, g, dtype), (g * x).to(dtype))
