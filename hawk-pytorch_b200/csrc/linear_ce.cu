@@ -103,6 +103,7 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t (&v)[32], int cbase
   }
   const float new_m = fmaxf(run_m, cmax);
   const float2 off = f2(-new_m * kLog2e);
+  const float err = fmaf(new_m, kLog2e, off.x);  // off's rounding, exactly: every term below carries the factor 2^err
   float2 add = f2(0.f);
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
@@ -111,7 +112,7 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t (&v)[32], int cbase
     t.y = ex2_approx(t.y);
     add = add2(add, t);
   }
-  run_s = fmaf(run_s, ex2_approx((run_m - new_m) * kLog2e), add.x + add.y);
+  run_s = fmaf(run_s, ex2_approx((run_m - new_m) * kLog2e), (add.x + add.y) * fmaf(err, -0.69314718f, 1.f));  // 2^-err
   run_m = new_m;
   if (row_ok && label >= cbase && label < cbase + 32) {
     const int at = (int)(label - cbase);

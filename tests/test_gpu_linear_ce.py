@@ -243,3 +243,22 @@ def test_scaled(n, dtype):
     g = torch.tensor(1.7, device="cuda")
     for x in (flat[:n], flat[1:]):  # at an aligned and an odd address
         assert torch.equal(ops.scaled(x, g, dtype), (g * x).to(dtype))
+
+
+@pytest.mark.parametrize("shift", [0.0, 300.0, -1000.0])
+def test_loss_of_shifted_logits(shift):
+    """The loss does not depend on a shift common to a row's logits, and its error is that of rounding each row's log-sum-exp
+    to fp32 (half an ulp of the shift, independent from row to row), not one common to all rows."""
+    from hawk_b200 import fused_cross_entropy
+    N, H, V = 2000, 512, 8000
+    g = torch.Generator(device="cuda").manual_seed(0)
+    w = (torch.randn(V, H, generator=g, device="cuda") / math.sqrt(H)).bfloat16()
+    act = torch.randn(N, H, generator=g, device="cuda").bfloat16()
+    if shift:
+        w[:, 0], act[:, 0] = shift, 1.0
+    labels = torch.randint(0, V, (N,), generator=g, device="cuda")
+    want = float(torch.nn.functional.cross_entropy((act @ w.t()).double(), labels))  # from the same bf16 logits on
+    ulp = 2.0 ** (math.floor(math.log2(max(abs(shift), 9.0))) - 23)
+    # the mean of N roundings, at four standard deviations, and fp32 sums of N terms and of the loss itself (a few ulp of it)
+    bound = 4 * ulp / math.sqrt(12 * N) + 1.5e-6
+    assert abs(float(fused_cross_entropy(w, act, labels)) - want) <= bound
