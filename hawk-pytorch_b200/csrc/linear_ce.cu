@@ -637,6 +637,17 @@ extern "C" size_t hawk_linear_ce_workspace_bytes(int64_t N, int64_t H, int64_t V
   return ce_saved(N, H, V, HAWK_F32, HAWK_F32).total + hawk_linear_ce_scratch_bytes(N, H, V);
 }
 
+// one cast per fp32 operand, the logits GEMM and the two reductions, the pass that makes dprobs; then a GEMM and, where K is
+// split, a sum for each gradient, and the look at the status word
+extern "C" int hawk_linear_ce_kernels(int64_t N, int64_t H, int64_t V, int w_dtype, int a_dtype, int want_dw, int want_da) {
+  if (N < 1 || H < 1 || V < 1) return 0;
+  int n = (w_dtype == HAWK_F32) + (a_dtype == HAWK_F32) + 3;
+  if (want_dw || want_da) n += 2;
+  if (want_dw) n += plan_grad(V, H, N).splits > 1 ? 2 : 1;
+  if (want_da) n += plan_grad(N, H, V).splits > 1 ? 2 : 1;
+  return n;
+}
+
 extern "C" int hawk_linear_ce_fwd(const void* weight, const void* act, const int64_t* labels, float* loss, void* saved,
                                   size_t saved_bytes, void* scratch, size_t scratch_bytes, int64_t N, int64_t H, int64_t V,
                                   int w_dtype, int a_dtype, int want_grad, int* status, void* stream) {

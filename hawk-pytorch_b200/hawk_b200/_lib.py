@@ -78,6 +78,7 @@ SIGNATURES = {
     "hawk_linear_ce_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
     "hawk_linear_ce_saved_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int, c_int]),
     "hawk_linear_ce_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
+    "hawk_linear_ce_kernels": (c_int, [c_int64, c_int64, c_int64, c_int, c_int, c_int, c_int]),
     "hawk_linear_ce_fwd": (c_int, [_P] * 5 + [c_size_t, _P, c_size_t, c_int64, c_int64, c_int64, c_int, c_int, c_int, _P, _P]),
     "hawk_linear_ce_bwd": (c_int, [_P, _P, _P, c_size_t, _P, _P, c_int, _P, c_int, _P, c_size_t, c_int64, c_int64, c_int64,
                                    c_int, c_int, _P, _P]),

@@ -87,7 +87,7 @@ class _on:
             raise RuntimeError("hawk_b200: tensors must be on a CUDA device (there is no CPU path)")
         self.idx = t.device.index
         self.prev = None
-        self.name, self.kernels = name, kernels
+        self.name, self.kernels = name, kernels  # kernels: their number, or a call that gives it (made only when logging)
         self.stream = None
         self.start = None
 
@@ -97,7 +97,7 @@ class _on:
             self.prev = cur
             torch.cuda.set_device(self.idx)
         if LOG.enabled and self.name:
-            LOG.counts[self.name] = LOG.counts.get(self.name, 0) + self.kernels
+            LOG.counts[self.name] = LOG.counts.get(self.name, 0) + (self.kernels() if callable(self.kernels) else self.kernels)
             if LOG.timed and (LOG.only is None or self.name in LOG.only):
                 self.stream = torch.cuda.current_stream()
                 self.start = torch.cuda.Event(enable_timing=True)
@@ -906,6 +906,11 @@ def _ce_grads(weight, act, saved, grad_loss, dw, da):
                                       _status_word(act.device).data_ptr(), _stream(act)), "hawk_linear_ce_bwd")
 
 
+def _ce_kernels(weight, act, want_dw, want_da):
+    return _lib.load().hawk_linear_ce_kernels(act.shape[0], act.shape[1], weight.shape[0], _dt(weight), _dt(act), int(want_dw),
+                                              int(want_da))
+
+
 def _ce_operands(weight, act, labels=None):
     # operands of two types: act may lie at any address (a cast to the weight's type would have moved it)
     act = act.contiguous() if act.dtype == weight.dtype else _dense16(act)
@@ -921,9 +926,8 @@ def linear_ce(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor, wan
     backward's pass over them: N32760 H2048 V32000 11.46 ms, 11.42 with the gradients formed in the backward call."""
     weight, act, labels = _ce_operands(weight, act, labels)
     (V, H), N = weight.shape, act.shape[0]
-    casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
     want = want_dw or want_da
-    with _on(act, "linear_ce", 3 + casts + (2 + want_dw + want_da if want else 0)):
+    with _on(act, "linear_ce", lambda: _ce_kernels(weight, act, want_dw, want_da)):
         loss, saved = _ce_forward(weight, act, labels, want)
         dw = torch.empty((V, H) if want_dw else 0, dtype=torch.float32, device=act.device)
         da = torch.empty((N, H) if want_da else 0, dtype=torch.float32, device=act.device)
@@ -983,8 +987,7 @@ def linear_ce_fwd(weight: torch.Tensor, act: torch.Tensor, labels: torch.Tensor,
                   want_grad: bool) -> Tuple[torch.Tensor, torch.Tensor]:
     """(loss [], saved): mean CE(act @ weight^T, labels) and, with want_grad, what linear_ce_bwd needs."""
     weight, act, labels = _ce_operands(weight, act, labels)
-    casts = (weight.dtype == torch.float32) + (act.dtype == torch.float32)
-    with _on(act, "linear_ce_fwd", 3 + casts + bool(want_grad)):
+    with _on(act, "linear_ce_fwd", lambda: _ce_kernels(weight, act, False, False) + bool(want_grad)):
         return _ce_forward(weight, act, labels, want_grad)
 
 
@@ -1006,7 +1009,7 @@ def linear_ce_bwd(weight: torch.Tensor, act: torch.Tensor, saved: torch.Tensor, 
     g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
     dw = torch.empty(weight.shape if want_dw else 0, dtype=weight.dtype, device=act.device)
     da = torch.empty(act.shape if want_da else 0, dtype=act.dtype, device=act.device)
-    with _on(act, "linear_ce_bwd", 1 + want_dw + want_da):
+    with _on(act, "linear_ce_bwd", lambda: _ce_kernels(weight, act, want_dw, want_da) - _ce_kernels(weight, act, False, False) - 1):
         _ce_grads(weight, act, saved, g, dw if want_dw else None, da if want_da else None)
     return dw, da
 

@@ -263,6 +263,8 @@ size_t hawk_linear_ce_workspace_bytes(int64_t N, int64_t H, int64_t V);
  * call.  An abandoned wait makes the loss, or the first element of each gradient, NaN. */
 size_t hawk_linear_ce_saved_bytes(int64_t N, int64_t H, int64_t V, int w_dtype, int a_dtype);
 size_t hawk_linear_ce_scratch_bytes(int64_t N, int64_t H, int64_t V);
+/* Kernels that the two calls launch together on the current device (with neither gradient: the first alone). */
+int hawk_linear_ce_kernels(int64_t N, int64_t H, int64_t V, int w_dtype, int a_dtype, int want_dw, int want_da);
 int hawk_linear_ce_fwd(const void* weight, const void* act, const int64_t* labels, float* loss, void* saved,
                        size_t saved_bytes, void* scratch, size_t scratch_bytes, int64_t N, int64_t H, int64_t V,
                        int w_dtype, int a_dtype, int want_grad, int* status, void* stream);

@@ -262,3 +262,31 @@ def test_loss_of_shifted_logits(shift):
     # the mean of N roundings, at four standard deviations, and fp32 sums of N terms and of the loss itself (a few ulp of it)
     bound = 4 * ulp / math.sqrt(12 * N) + 1.5e-6
     assert abs(float(fused_cross_entropy(w, act, labels)) - want) <= bound
+
+
+# K unsplit in both gradient GEMMs, split in one, split in both; each gradient alone, bf16 operands
+@pytest.mark.parametrize("N,H,V", [(60, 64, 64), (513, 264, 1031), (300, 72, 5000), (4000, 520, 9000)])
+@pytest.mark.parametrize("dtype,which", [(torch.float32, (0, 1)), (torch.bfloat16, (0, 1)), (torch.float32, (0,)), (torch.float32, (1,)),
+                                         (torch.float32, ())])
+def test_launches_are_counted(N, H, V, dtype, which):
+    """What LOG counts for the loss is what a profiler sees of this library's kernels."""
+    from hawk_b200 import fused_cross_entropy, ops
+    w, act, labels = _case(N, H, V, seed=6)
+    t = [w.to("cuda", dtype), act.to("cuda", dtype)]
+    for i in which:
+        t[i].requires_grad_()
+    labels = labels.cuda()
+
+    def step():
+        loss = fused_cross_entropy(*t, labels)
+        if which:
+            torch.autograd.grad(loss, [t[i] for i in which])
+    step()
+    torch.cuda.synchronize()
+    ops.LOG.reset()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        step()
+        torch.cuda.synchronize()
+    counted = ops.LOG.total_launches()
+    ops.LOG.reset(enabled=False)
+    assert counted == sum(e.count for e in prof.key_averages() if "hawk::" in e.key)
