@@ -165,10 +165,10 @@ def main(argv=None):
         _emit("add_rms_norm_fwd", tf, (8 + 2 * es) * N * a.H, "GB/s", N=N, H=a.H, dtype=a.dtype)
         _emit("add_rms_norm_bwd", tb, (12 + 2 * es) * N * a.H, "GB/s", N=N, H=a.H, dtype=a.dtype)
     elif a.op == "linear_ce":
-        w = torch.randn(a.V, a.H, generator=g, device=dev) / math.sqrt(a.H)
-        act = torch.randn(a.N, a.H, generator=g, device=dev)
+        w = (torch.randn(a.V, a.H, generator=g, device=dev) / math.sqrt(a.H)).requires_grad_()
+        act = torch.randn(a.N, a.H, generator=g, device=dev).requires_grad_()
         lab = torch.randint(0, a.V, (a.N,), generator=g, device=dev)
-        t = _time(lambda: ops.linear_ce(w, act, lab), max(3, a.iters // 4), 2, flush)
+        t = _time(lambda: torch.autograd.grad(ops.fused_cross_entropy(w, act, lab), (w, act)), max(3, a.iters // 4), 2, flush)
         ops.check_device_status()
         _emit("linear_ce", t, 6 * a.N * a.H * a.V, "TFLOP/s", N=a.N, H=a.H, V=a.V)
     elif a.op == "decode_model":
