@@ -340,10 +340,10 @@ def chain_rows(fp32_weights: bool) -> int:
 
 
 def _chain_ok(hidden: torch.Tensor) -> Optional[bool]:
-    """Whether a cached token's activations [B, 1, H] are ones the chained decode kernels take: bf16 ones,
-    for at most 256 rows and outside autograd and tracing.  None if not; otherwise whether bf16 autocast is on."""
+    """Whether a cached token's activations [B, 1, H] are ones the chained decode kernels take: bf16 ones, outside autograd
+    and tracing (chain_rows says for how many rows).  None if not; otherwise whether bf16 autocast is on."""
     if (not hidden.is_cuda or torch.is_grad_enabled() or torch.compiler.is_compiling() or hidden.dim() != 3
-            or hidden.shape[1] != 1 or not 1 <= hidden.shape[0] <= 256 or hidden.shape[2] % 8 or hidden.shape[2] > 8192
+            or hidden.shape[1] != 1 or hidden.shape[0] < 1 or hidden.shape[2] % 8 or hidden.shape[2] > 8192
             or type(hidden) is not torch.Tensor or _any_global_hooks()):
         return None
     if torch.is_autocast_enabled("cuda"):

@@ -196,7 +196,7 @@ int hawk_decode_block_step(const void* xy, int64_t xy_row_stride, void* conv_sta
  * with a type of its own; gate weights and the caches as in hawk_decode_block_step.  H, R, I multiples of 8, H <= 8192; all
  * pointers 16-byte aligned; nothing may be written elsewhere while the call's kernels run;
  * follows_layer: the kernel before this call on the stream is that of another hawk_decode_layer, so that w_xy may be read
- * before it has ended.  Waits are bounded: `status` as in
+ * before it has ended.  Made for few rows: past 64 the same steps as separate calls are faster.  Waits are bounded: `status` as in
  * hawk_linear_ce_fwd_bwd, and the results of a launch that gave up are NaN. */
 typedef struct hawk_decode_layer_args {
   const void *residual, *pending;

@@ -6,7 +6,7 @@ import torch
 import hawk_b200.ops as ops
 from conftest import rel_l2
 from hawk_b200.generate import GraphedDecoder
-from hawk_b200.model import HawkConfig, HawkModel
+from hawk_b200.model import HawkConfig, HawkModel, Linear
 
 pytestmark = pytest.mark.gpu
 
@@ -117,3 +117,38 @@ def test_cached_token_after_replaced_weights(how):
             p.data = state[k]
     for a, b in zip(run(model), run(other)):
         assert torch.equal(a, b)
+
+
+# an fp32 residual with bf16 weights, as decoding under autocast has it once an optimiser has left bf16 copies: both kernels, a
+# ragged group of each size, K at and past 512 and in more than one step
+@pytest.mark.parametrize("rows", [1, 8, 11, 16, 17])
+@pytest.mark.parametrize("H,N", [(256, 136), (512, 200), (520, 264), (2048, 768), (4096, 136)])
+@pytest.mark.parametrize("wdt,rdt", [(torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+def test_norm_linear_of_mixed_types(rows, H, N, wdt, rdt):
+    test_norm_linear(rows, H, N, wdt, rdt)
+
+
+@pytest.mark.parametrize("hidden,inter,blocks,batch", [(64, 72, 4, 3), (256, 768, 16, 13), (256, 768, 16, 19), (1024, 3072, 16, 2)])
+def test_cached_token_with_bf16_copies(hidden, inter, blocks, batch):
+    """Under autocast, with the bf16 copies that FusedAdamW leaves on the projections: the chain reads them and its results
+    are those of the modules."""
+    torch.manual_seed(hidden + batch)
+    model = _model(1000, hidden, inter, 2, blocks)
+    for m in model.modules():
+        if isinstance(m, Linear):
+            m.weight_bf16, m.weight_bf16_version = m.weight.detach().bfloat16(), m.weight._version
+    dec = GraphedDecoder(model, batch, use_graph=False)
+    ids = torch.randint(0, 1000, (batch, 6), device="cuda")
+    outs = []
+    for hooked in (False, True):
+        handles = [m.register_forward_hook(lambda *_: None) for m in model.modules() if isinstance(m, torch.nn.Linear)] if hooked else []
+        dec.prefill(ids[:, :4])
+        ops.LOG.reset()
+        outs.append([dec.step(ids[:, t:t + 1]) for t in (4, 5)])
+        assert ("decode_layer" in ops.LOG.counts) == (not hooked)
+        ops.LOG.reset(enabled=False)
+        for h in handles:
+            h.remove()
+    for a, b in zip(*outs):
+        assert a.dtype == b.dtype and rel_l2(a, b) < 2e-2
+    ops.check_device_status()
