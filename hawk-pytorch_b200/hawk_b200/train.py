@@ -54,29 +54,39 @@ class FusedAdamW(torch.optim.Optimizer):
         for group in self.param_groups:
             b1, b2 = group["betas"]
             lr, eps, wd = group["lr"], group["eps"], group["weight_decay"]
-            batches = {}  # (device, step) -> the addresses of its tensors, as hawk_adamw_tensor lays them out
-            for p in group["params"]:
-                g = p.grad
-                if g is None:
-                    continue
-                st = self.state[p]
-                if not st:
-                    self._init_state(p, st)
-                st["step"] += 1
-                if not g.is_contiguous():
-                    g = g.contiguous()
-                    keep.append(g)
-                if st["_args"][0] != p.data_ptr():  # the parameter was moved or re-allocated since the state was made
-                    self._bind(p, st)
-                p_ptr, m_ptr, v_ptr, wb_ptr, n, dev = st["_args"]
-                batches.setdefault((dev, st["step"]), []).extend((p_ptr, g.data_ptr(), m_ptr, v_ptr, wb_ptr or 0, n))
-                touched.append(p)
-            for (dev, step), flat in batches.items():
-                with torch.cuda.device(dev):
-                    rc = lib.hawk_adamw_multi(struct.pack(f"{len(flat)}Q", *flat), len(flat) // 6, lr, b1, b2, eps, wd, step,
-                                              torch.cuda.current_stream().cuda_stream)
-                _lib.check(rc, "hawk_adamw_multi")
-                launches += (len(flat) // 6 + 63) // 64
+            # (device, step) -> the addresses of its tensors, as hawk_adamw_tensor lays them out, and their states
+            batches = {}
+            try:
+                for p in group["params"]:
+                    g = p.grad
+                    if g is None:
+                        continue
+                    st = self.state[p]
+                    if not st:
+                        self._init_state(p, st)
+                    if not g.is_contiguous():
+                        g = g.contiguous()
+                        keep.append(g)
+                    if st["_args"][0] != p.data_ptr():  # the parameter was moved or re-allocated since the state was made
+                        self._bind(p, st)
+                    p_ptr, m_ptr, v_ptr, wb_ptr, n, dev = st["_args"]
+                    st["step"] += 1
+                    flat, states = batches.setdefault((dev, st["step"]), ([], []))
+                    flat.extend((p_ptr, g.data_ptr(), m_ptr, v_ptr, wb_ptr or 0, n))
+                    states.append(st)
+                    touched.append(p)
+                for (dev, step), (flat, states) in batches.items():
+                    with torch.cuda.device(dev):
+                        rc = lib.hawk_adamw_multi(struct.pack(f"{len(flat)}Q", *flat), len(flat) // 6, lr, b1, b2, eps, wd, step,
+                                                  torch.cuda.current_stream().cuda_stream)
+                    _lib.check(rc, "hawk_adamw_multi")
+                    launches += (len(flat) // 6 + 63) // 64
+                    states.clear()
+            except BaseException:
+                for _, states in batches.values():  # counted, not updated
+                    for st in states:
+                        st["step"] -= 1
+                raise
         if touched:
             torch.autograd.graph.increment_version(touched)  # the kernels wrote p behind autograd's back
             for p in touched:

@@ -108,3 +108,23 @@ def test_fused_adamw_many_tensors_around_its_chunks():
         o2.step()
     for a, b in zip(mine, ref):  # the bound of the test above
         assert float((a - b).abs().max()) <= 2e-6 * float(b.abs().max())
+
+
+def test_a_step_that_fails_is_not_counted():
+    """A parameter that FusedAdamW refuses, after others of its group: nothing was updated, so nothing may have been counted
+    (the bias correction of the next step would be that of a second one)."""
+    from hawk_b200.train import FusedAdamW
+    torch.manual_seed(0)
+    good = torch.nn.Parameter(torch.randn(300, device="cuda"))
+    bad = torch.nn.Parameter(torch.randn(8, device="cuda", dtype=torch.bfloat16))
+    same = torch.nn.Parameter(good.detach().clone())
+    opt, ref = FusedAdamW([good, bad], lr=1e-2), torch.optim.AdamW([same], lr=1e-2)
+    good.grad, bad.grad, same.grad = torch.randn_like(good), torch.randn_like(bad), None
+    same.grad = good.grad.clone()
+    with pytest.raises(AssertionError):
+        opt.step()
+    assert torch.equal(good, same) and opt.state[good]["step"] == 0
+    bad.grad = None
+    opt.step()
+    ref.step()
+    assert opt.state[good]["step"] == 1 and torch.allclose(good, same, rtol=1e-6, atol=1e-7)
