@@ -309,9 +309,14 @@ class Hawk(nn.Module):
 
 
 # ---- a cached token's layer as one chain of launches ---------------------------------------------------
+_METHODS = frozenset(("forward", "step", "add_forward", "_decode", "_fp32", "_weight32"))
+
+
 def _plain(module: nn.Module, kind: type) -> bool:
-    """Exactly the module class written here and nothing hooked into its call: it may be replaced by what it computes."""
-    return type(module) is kind and not (module._forward_hooks or module._forward_pre_hooks or "forward" in module.__dict__)
+    """Exactly the module class written here, nothing hooked into its call and none of its methods replaced on the object: it
+    may be replaced by what it computes."""
+    return (type(module) is kind and not (module._forward_hooks or module._forward_pre_hooks)
+            and _METHODS.isdisjoint(module.__dict__))
 
 
 def _any_global_hooks() -> bool:
@@ -441,7 +446,8 @@ class HawkModel(nn.Module):
         caches = []
         chained = False
         for layer, past in zip(self.layers, layer_past):
-            done = layer._decode_chain(hidden, pending, past, chained) if type(layer) is RNNLayer else None
+            own_step = type(layer) is RNNLayer and "step" not in layer.__dict__
+            done = layer._decode_chain(hidden, pending, past, chained) if own_step else None
             chained = done is not None
             hidden, pending, cache = (*done, past) if chained else layer.step(hidden, pending, past)
             caches.append(cache)

@@ -152,3 +152,20 @@ def test_cached_token_with_bf16_copies(hidden, inter, blocks, batch):
     for a, b in zip(*outs):
         assert a.dtype == b.dtype and rel_l2(a, b) < 2e-2
     ops.check_device_status()
+
+
+def test_methods_replaced_on_an_object_are_called():
+    """A layer's `step`, or a method of one of its modules, replaced on the object: a cached token calls it too."""
+    torch.manual_seed(1)
+    model = _model(500, 128, 256, 2, 4).bfloat16()
+    ids = torch.randint(0, 500, (3, 6), device="cuda")
+    dec = GraphedDecoder(model, 3, autocast=False, use_graph=False)
+    for module, name in [(model.layers[1], "step"), (model.layers[0].input_norm, "add_forward"), (model.norm, "add_forward"),
+                         (model.layers[0].recc, "_decode")]:
+        calls, own = [], getattr(module, name)
+        setattr(module, name, lambda *args, own=own, calls=calls: (calls.append(1), own(*args))[1])
+        dec.prefill(ids[:, :4])
+        calls.clear()
+        dec.step(ids[:, 4:5])
+        assert len(calls) == 1, name
+        delattr(module, name)
