@@ -626,9 +626,17 @@ class Conv1D(nn.Module):
 # ---------------------------------------------------------------------------------------------
 # cached decode step
 # ---------------------------------------------------------------------------------------------
+def _same_device(t: torch.Tensor, *others: Optional[torch.Tensor]) -> None:
+    """The caches are the caller's own objects: one left on another device would reach the kernel as an address it cannot read."""
+    for o in others:
+        if o is not None and o.device != t.device:
+            raise RuntimeError(f"hawk_b200: tensors on {t.device} and {o.device} in one call")
+
+
 @_operator("hawk_b200::decode_conv_step", mutates_args=("conv_state",))
 def decode_conv_step(x_new: torch.Tensor, conv_state: torch.Tensor, w: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """x_new [B,D] (row-strided ok), conv_state [B,W-1,D] contiguous, rolled in place. Returns y [B,D]."""
+    _same_device(x_new, conv_state, w, b)
     lib = _lib.load()
     B, D = x_new.shape
     if x_new.stride(1) != 1 or x_new.stride(0) % 8 or x_new.data_ptr() % 16:
@@ -654,6 +662,7 @@ def decode_block_step(xy: torch.Tensor, conv_state: torch.Tensor, conv_w: torch.
     """One cached token through the whole recurrent branch in one launch: xy [B,2R] = [x_b | y] (row-strided
     ok), conv_state [B,W-1,R] and state [B,R] updated in place, gate weights [nb,bw,bw] (fp32 or bf16),
     biases / conv taps / Lambda fp32.  Returns gelu(y) * h, [B,R] in xy's dtype."""
+    _same_device(xy, conv_state, conv_w, conv_b, wx, wa, bx, ba, lam, state)
     lib = _lib.load()
     B, R2 = xy.shape
     R = R2 // 2
@@ -682,6 +691,7 @@ def _(xy, conv_state, conv_w, conv_b, wx, wa, bx, ba, lam, state):
 def decode_rglru_step(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Tensor,
                       state: torch.Tensor) -> torch.Tensor:
     """One recurrence step on [B,D]; `state` is overwritten with h; returns h in x's dtype."""
+    _same_device(x, gx, ga, lam, state)
     lib = _lib.load()
     B, D = x.shape
     x, gx, ga = x.contiguous(), gx.contiguous(), ga.contiguous()
@@ -702,6 +712,7 @@ def _(x, gx, ga, lam, state):
 @_operator("hawk_b200::core_params", mutates_args=())
 def core_params(conv_w: torch.Tensor, conv_b: torch.Tensor, bx: torch.Tensor, ba: torch.Tensor, lam: torch.Tensor) -> torch.Tensor:
     """fp32 values of conv_w [W,R], conv_b [R], the gate biases [nb,bw] and Lambda [R], one after the other."""
+    _same_device(conv_w, conv_b, bx, ba, lam)
     lib = _lib.load()
     W, R = conv_w.shape
     assert conv_b.numel() == bx.numel() == ba.numel() == lam.numel() == R
@@ -723,6 +734,7 @@ def _(conv_w, conv_b, bx, ba, lam):
 def cache_store(x: torch.Tensor, h: torch.Tensor, conv_state: torch.Tensor, state: torch.Tensor) -> None:
     """The decode caches after a prompt: conv_state [B,keep,R] takes the last rows of x [B,T,R] (zero before its first one;
     x may be row-strided), state [B,1,R] the last row of h [B,T,R]."""
+    _same_device(x, h, conv_state, state)
     lib = _lib.load()
     B, T, R = x.shape
     keep = conv_state.shape[1]
@@ -755,6 +767,7 @@ def decode_layer(residual: torch.Tensor, pending: Optional[torch.Tensor], norm1:
     """One cached token through a whole layer: (residual, pending) -> (residual, pending), [.., H] for up to 256 rows; norms,
     taps, biases and Lambda in fp32, projection weights fp32 (rounded to bf16 as they are read) or bf16, activations bf16.  follows_layer: nothing has run on the stream since
     the call for the layer before (its kernels and this one's may then overlap further)."""
+    _same_device(residual, pending, norm1, w_xy, conv_w, conv_b, wx, wa, bx, ba, lam, w_res, norm2, w_gu, w_down, conv_state, state)
     lib = _lib.load()
     H = residual.shape[-1]
     B, R, (nb, bw, _), I = residual.numel() // H, lam.numel(), wx.shape, w_down.shape[1]
@@ -795,6 +808,7 @@ def decode_norm_linear(residual: torch.Tensor, pending: Optional[torch.Tensor], 
                        weight: torch.Tensor, follows_layer: bool) -> torch.Tensor:
     """bf16 rms_norm(residual + pending) @ weight^T for up to 256 rows [.., H] (the final norm and the head of a cached token);
     `weight` [N, H] fp32 (rounded to bf16 as it is read) or bf16; follows_layer as in decode_layer."""
+    _same_device(residual, pending, norm, weight)
     lib = _lib.load()
     H, N = residual.shape[-1], weight.shape[0]
     B = residual.numel() // H

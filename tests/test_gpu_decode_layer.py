@@ -169,3 +169,15 @@ def test_methods_replaced_on_an_object_are_called():
         dec.step(ids[:, 4:5])
         assert len(calls) == 1, name
         delattr(module, name)
+
+
+@pytest.mark.parametrize("batch", [2, 40])  # the chained kernels, the modules
+def test_caches_on_another_device_are_refused(batch):
+    model = _model(500, 128, 256, 2, 4).bfloat16()
+    caches = model.new_caches(batch, device="cpu")
+    for c in caches:
+        c.recc_state.zero_()
+        c.conv_state.zero_()
+        c.current_cache_size = 1
+    with torch.no_grad(), pytest.raises(RuntimeError, match="tensors on cuda:0 and cpu"):
+        model(torch.zeros(batch, 1, dtype=torch.long, device="cuda"), layer_past=caches)
