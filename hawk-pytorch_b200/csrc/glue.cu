@@ -289,9 +289,9 @@ __device__ __forceinline__ float row_sum(float v, float (&part)[TPR / 32], int g
 // scaling, so the row is read once.  What bounds it is bytes in flight: a thread's loads of one row are all it has
 // outstanding.  With 128 threads to a row of 512 that was one 16-byte load per tensor (N32768, fp32 stream, bf16 branch:
 // 42.2 us forward, 60.3 us backward, 4.8 and 4.4 TB/s); a warp to a row has four of each.  Groups are the narrowest that
-// keep a row's state in registers (NCH = 4), 128 threads from H = 1536 on.
+// keep a row's state in few registers (NCH <= 4), up to eight vectors where no such group divides the row.
 template <typename TX, typename TY, int TPR, int NCH>
-__global__ void __launch_bounds__(256, (NCH >= 8 ? 2 : 3))
+__global__ void __launch_bounds__(256, (NCH >= 6 ? 2 : 3))
 rms_norm_fwd_rows_kernel(const TX* __restrict__ x, const TY* __restrict__ delta, TX* __restrict__ x_out,
                          const float* __restrict__ w, TY* __restrict__ y, float* __restrict__ rstd, int64_t M,
                          float eps) {
@@ -428,7 +428,7 @@ rms_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, const f
 // per thread at NCH = 4) are in flight together, and w is loaded once per thread because a thread keeps its columns for
 // every row.  dw partials: per-thread column sums, the CTA's groups added in shared memory, one partial row per CTA.
 template <typename TX, typename TY, int TPR, int NCH>
-__global__ void __launch_bounds__(256, (NCH >= 8 ? 1 : 2))
+__global__ void __launch_bounds__(256, (NCH >= 6 ? 1 : 2))
 rms_norm_bwd_rows_kernel(const TY* __restrict__ dy, const TX* __restrict__ x, const float* __restrict__ w,
                          const float* __restrict__ rstd, const TX* __restrict__ gres, TX* __restrict__ dx,
                          TY* __restrict__ ddelta, float* __restrict__ dw_partial, int64_t M) {
@@ -648,21 +648,54 @@ extern "C" int hawk_gelu_mul_bwd(const void* dout, int64_t ldd, const void* a, i
   return launch_status();
 }
 
-// widths of the rows-in-registers kernels; any other H takes the warp-per-row kernels, which read a row twice
-static bool norm_rows_width(int H) {
-  return H == 256 || H == 512 || H == 768 || H == 1024 || H == 1536 || H == 2048 || H == 4096;
+// Threads to a row (TPR) and 16-byte vectors per thread (NCH) of the rows-in-registers kernels, as TPR * 16 + NCH, or 0 for a
+// width that the warp-per-row kernels take, which read a row twice.  Any H = 4 * TPR * NCH has a form; of several the one with
+// the narrowest group that needs no more than four vectors (see rms_norm_fwd_rows_kernel), else the widest with at most eight.
+static int norm_rows_form(int H) {
+  int form = 0;
+  for (int tpr = 32; tpr <= 128; tpr *= 2) {
+    const int nch = H / (4 * tpr);
+    if (nch * 4 * tpr != H || nch < 1 || nch > 8) continue;
+    form = tpr * 16 + nch;
+    if (nch <= 4) break;
+  }
+  return form;
 }
-#define HAWK_NORM_WIDTHS(LAUNCH, TX, TY)          \
-  do {                                            \
-    switch (H) {                                  \
-      case 256: LAUNCH(TX, TY, 32, 2); break;     \
-      case 512: LAUNCH(TX, TY, 32, 4); break;     \
-      case 768: LAUNCH(TX, TY, 64, 3); break;     \
-      case 1024: LAUNCH(TX, TY, 64, 4); break;    \
-      case 1536: LAUNCH(TX, TY, 128, 3); break;   \
-      case 2048: LAUNCH(TX, TY, 128, 4); break;   \
-      default: LAUNCH(TX, TY, 128, 8); break;     \
-    }                                             \
+// Whether the forward takes its form.  Up to some thousand rows, where latency counts, it always is the faster one; with the
+// grid full it is bytes in flight that count, and a bf16 stream, 8 bytes to a thread's vector, has enough of them only in forms
+// of four and eight vectors.  us, warp per row / rows in registers, x and branch as given:
+//                   bf16, bf16                                   fp32, bf16               fp32, fp32
+//   H       M 1551      3108       8192       32768      M 3108     32768         M 3108     32768
+//   128     8.1 / 8.2                         14 / 21    8.2 / 8.2  16 / 18       8.2 / 8.2  18 / 19
+//   256     8.2 / 8.2   8.2 / 8.2  10 / 12    21 / 23    9.2 / 8.2  26 / 25       10 / 8     31 / 29
+//   384     8.2 / 8.2   10 / 8     12 / 12    25 / 29    10 / 10    32 / 31       10 / 10    39 / 41
+//   768     11 / 8      12 / 10    16 / 18    41 / 49    12 / 12    55 / 55       14 / 12    69 / 72
+//   1280    14 / 10     15 / 12    23 / 23    64 / 64    16 / 14    90 / 88       19 / 16    111 / 115
+//   1536    16 / 10     17 / 15    25 / 29    76 / 90    19 / 16    107 / 100     21 / 20    133 / 135
+//   2048    19 / 12     21 / 16    33 / 33    104 / 103  23 / 19    150 / 135     27 / 23    186 / 179
+//   3072    25 / 16     29 / 25    51 / 53    164 / 188  33 / 27    248 / 203     39 / 32    305 / 258
+//   4096    33 / 18     37 / 29    67 / 61    226 / 221  47 / 32    342 / 262     53 / 39    418 / 341
+// The backward is faster in every form (32768 rows, fp32 stream, bf16 branch: 128 36 / 28, 384 75 / 44, 768 124 / 75, 1280
+// 190 / 120, 2048 292 / 177, 3072 546 / 265).
+static bool norm_fwd_in_rows(int form, int64_t M, int x_dtype) {
+  const int nch = form % 16;
+  return form != 0 && (M <= 4096 || nch % 4 == 0 || (x_dtype == HAWK_F32 && nch >= 2));
+}
+#define HAWK_NORM_FORM(LAUNCH, TX, TY, TPR, NCH) \
+  case TPR * 16 + NCH: LAUNCH(TX, TY, TPR, NCH); break
+#define HAWK_NORM_WIDTHS(LAUNCH, TX, TY)                                                          \
+  do {                                                                                            \
+    switch (norm_rows_form(H)) {                                                                  \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 32, 1);  HAWK_NORM_FORM(LAUNCH, TX, TY, 32, 2);              \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 32, 3);  HAWK_NORM_FORM(LAUNCH, TX, TY, 32, 4);              \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 32, 5);  HAWK_NORM_FORM(LAUNCH, TX, TY, 32, 7);              \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 64, 3);  HAWK_NORM_FORM(LAUNCH, TX, TY, 64, 4);              \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 64, 5);  HAWK_NORM_FORM(LAUNCH, TX, TY, 64, 7);              \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 128, 3); HAWK_NORM_FORM(LAUNCH, TX, TY, 128, 4);             \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 128, 5); HAWK_NORM_FORM(LAUNCH, TX, TY, 128, 6);             \
+      HAWK_NORM_FORM(LAUNCH, TX, TY, 128, 7); HAWK_NORM_FORM(LAUNCH, TX, TY, 128, 8);             \
+      default: return HAWK_ERR_UNSUPPORTED; /* a form without an instance: norm_rows_form gave none of these */ \
+    }                                                                                             \
   } while (0)
 
 static int norm_fwd_impl(const void* x, const void* delta, void* x_out, const float* w, void* y, float* rstd,
@@ -672,7 +705,7 @@ static int norm_fwd_impl(const void* x, const void* delta, void* x_out, const fl
   HAWK_REQUIRE(M >= 1 && H >= 4 && H % 4 == 0, HAWK_ERR_SHAPE);
   HAWK_REQUIRE(aligned(x, 16) && aligned(w, 16) && aligned(y, 16) && aligned(delta, 16) && aligned(x_out, 16),
                HAWK_ERR_ALIGN);
-  if (norm_rows_width(H)) {  // rows-in-registers path
+  if (norm_fwd_in_rows(norm_rows_form(H), M, x_dtype)) {  // rows-in-registers path
 #define HAWK_NORM_FROWS_N(TX, TY, TPR, N)                                                                                  \
   rms_norm_fwd_rows_kernel<TX, TY, TPR, N><<<(unsigned)std::min<int64_t>((M + 256 / TPR - 1) / (256 / TPR), 148 * 3), 256, 0, st>>>( \
       static_cast<const TX*>(x), static_cast<const TY*>(delta), static_cast<TX*>(x_out), w, static_cast<TY*>(y), rstd, M, eps)
@@ -724,7 +757,7 @@ static int norm_bwd_impl(const void* dy, const void* x, const float* w, const fl
                    aligned(gres, 16) && aligned(ddelta, 16),
                HAWK_ERR_ALIGN);
   float* partial = static_cast<float*>(workspace);
-  if (norm_rows_width(H)) {  // rows-in-registers path
+  if (norm_rows_form(H)) {  // rows-in-registers path
 #define HAWK_NORM_ROWS_N(TX, TY, TPR, N)                                                                              \
   rms_norm_bwd_rows_kernel<TX, TY, TPR, N><<<kNormBwdCtas, 256, 0, st>>>(                                                  \
       static_cast<const TY*>(dy), static_cast<const TX*>(x), w, rstd, static_cast<const TX*>(gres),                   \

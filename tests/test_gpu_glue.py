@@ -275,3 +275,29 @@ def test_drop_last(B, T, H, dt):
     assert out.is_contiguous() and torch.equal(out, x[:, :-1])
     dx, = torch.autograd.grad(out, x, go)
     assert torch.equal(dx, torch.nn.functional.pad(go, (0, 0, 0, 1)))
+
+
+@pytest.mark.parametrize("xdt,ydt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16),
+                                     (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("H", [128, 384, 640, 896, 1152, 1280, 1792, 2560, 3072, 3584])
+def test_add_rms_norm_widths(xdt, ydt, H):
+    """Every form of the rows-in-registers kernels that the widths above do not reach, and a multiple of 128 without one
+    (1152), with the residual add and its gradient; fewer rows than a CTA's groups, more than one pass of the grid, and more
+    rows than the forward's line for a bf16 stream."""
+    from hawk_b200 import ops
+    for M in (3, 4000, 4100):
+        g = torch.Generator().manual_seed(M + H)
+        x, gr = ((3 * torch.randn(M, H, generator=g)).to(xdt) for _ in range(2))
+        d, go = (torch.randn(M, H, generator=g).to(ydt) for _ in range(2))
+        w = 1 + 0.1 * torch.randn(H, generator=g)
+        xs, y, rstd = ops.add_rms_norm_fwd(x.cuda(), d.cuda(), w.cuda(), 1e-6, ydt)
+        s = (x.float() + d.float()).to(xdt)
+        assert torch.equal(xs.cpu(), s)
+        sr, wr = s.double().requires_grad_(), w.double().requires_grad_()
+        ref = sr * torch.rsqrt(sr.pow(2).mean(-1, keepdim=True) + 1e-6) * wr
+        ref.backward(go.double())
+        dres, ddelta, dw = ops.add_rms_norm_bwd(gr.cuda(), go.cuda(), xs, w.cuda(), rstd)
+        assert rel_l2(y.float().cpu(), ref.detach()) <= _tol(ydt)
+        assert rel_l2(dres.float().cpu(), sr.grad + gr.double()) <= _tol(xdt if xdt == ydt else ydt)
+        assert rel_l2(ddelta.float().cpu(), sr.grad + gr.double()) <= _tol(ydt)
+        assert rel_l2(dw.cpu(), wr.grad) <= (1e-5 if ydt == torch.float32 else 2e-2)
