@@ -1112,11 +1112,33 @@ static int split_view(const void* p, int64_t bs, int64_t ld, int T, int L, int D
 
 extern "C" int hawk_scan_split_chunks(int B, int T, int D, int pass) {
   if (B < 1 || T < 1 || D < 64) return 1;
-  // CTAs of the whole-sequence launch at its narrowest shape: 16 channels per CTA for the plain forward, 32 for
-  // the forward with the epilogue and for the backward.  Measured on B200 (bf16, T = 65536): with 64 such CTAs
-  // the split is 1.5-1.7x faster (the plain forward at 128 CTAs is not: 0.35 against 0.38 ms), with 16 CTAs
-  // 2.9-5.7x; at 128 CTAs the whole-sequence kernels already run at 4.4 TB/s and reading twice costs more.
-  if ((int64_t)B * (D / (pass == HAWK_SCAN_PASS_FWD ? 16 : 32)) > 64) return 1;
+  // A whole-sequence launch with few groups of 32 channels (g = B D / 32) takes a time that goes with T alone; a split one starts
+  // three to five kernels and reads its inputs twice, a time that goes with g T.  Measured on B200, L2 flushed, us, whole / split:
+  //                     bf16, plain fwd   bwd          fused fwd   fused bwd    fp32, plain fwd   bwd          fused fwd    fused bwd
+  //   T 1024   g  2     12 / 17           26 / 28      19 / 17     30 / 30      23 / 26           32 / 46      39 / 30      65 / 42
+  //            g 32     13 / 21           28 / 34      19 / 24     32 / 34      25 / 32           36 / 40      41 / 36      69 / 48
+  //            g 64     14 / 24           28 / 36      20 / 26     34 / 40      27 / 40           38 / 48      42 / 50      71 / 58
+  //   T 2048   g  2     18 / 19           42 / 30      31 / 19     50 / 32      41 / 28           60 / 48      74 / 32      124 / 44
+  //            g 32     18 / 24           44 / 36      31 / 26     52 / 40      41 / 40           59 / 48      74 / 52      126 / 58
+  //            g 48     18 / 28           44 / 46      31 / 30     52 / 52      41 / 52           60 / 73      74 / 64      126 / 81
+  //   T 4096   g  8     29 / 21           73 / 34      53 / 23     89 / 36      74 / 32           99 / 42      139 / 36     234 / 50
+  //            g 24     29 / 28           73 / 48      55 / 30     91 / 52      74 / 52           101 / 73     140 / 65     235 / 81
+  //            g 64     31 / 40           75 / 62      55 / 48     91 / 77      76 / 93           103 / 116    140 / 128    239 / 142
+  //   T 8192   g 32     49 / 42           132 / 65     100 / 47    169 / 79     141 / 93          189 / 118    272 / 126    464 / 144
+  //            g 48     49 / 58           134 / 89     100 / 71    169 / 108    141 / 142         189 / 175    272 / 179    466 / 219
+  //            g 64     51 / 67           134 / 99     100 / 77    169 / 124    141 / 157         191 / 196    272 / 220    464 / 251
+  //   T 65536  g 64     346 / 390         970 / 580    751 / 486   1251 / 755   1068 / 1062       1416 / 1311  2119 / 1519  3625 / 1769
+  //            g 96     508 / 622         854 / 918    688 / 757   1119 / 1207  1276 / 1929       1836 / 2286  2500 / 2495  3629 / 2988
+  const int64_t g = (int64_t)B * (D / 32);
+  const bool f32 = (pass & HAWK_SCAN_PASS_F32) != 0;
+  const int which = pass & ~HAWK_SCAN_PASS_F32;
+  const bool fused = which == HAWK_SCAN_PASS_FWD_GELU || which == HAWK_SCAN_PASS_BWD_GELU;
+  if (g > (which == HAWK_SCAN_PASS_FWD ? 32 : 64)) return 1;
+  int64_t least = 1024 + 32 * g;                                    // of T
+  if (f32 && fused) least = 1024;                                   // the slowest whole-sequence kernels
+  if (!f32 && which == HAWK_SCAN_PASS_FWD) least = 2048 + 128 * g;  // the fastest
+  if (f32 && which == HAWK_SCAN_PASS_BWD && g > 32) least = 128 * g;  // past L2, where the second reading costs
+  if (T < least) return 1;
   const int64_t ctas = (int64_t)B * (D / 32);  // per sub-sequence in the split launches
   const int want = (int)std::min<int64_t>((2 * 148 + ctas - 1) / ctas, kSplitMaxSub);
   for (int n = want; n <= kSplitMaxSub; ++n)

@@ -224,6 +224,11 @@ def _operator(name, mutates_args):
 SCAN_BYTES_PER_ELEMENT = {"scan_fwd": 8, "scan_bwd": 16, "scan_gelu_fwd": 12, "scan_gelu_bwd": 20}
 SCAN_ENTRY_POINTS = ("scan_gelu_fwd", "scan_gelu_bwd")
 
+def _split_chunks(lib, x, which):
+    """Pieces to cut the sequences of x [B,T,D] into for a pass: 0 / 2 the plain forward / backward, 1 / 3 with the epilogue."""
+    return lib.hawk_scan_split_chunks(*x.shape, which + (8 if x.dtype == torch.float32 else 0))
+
+
 def _split_workspace(lib, x, B, nsub, D):
     return torch.empty(lib.hawk_scan_split_workspace_bytes(B, nsub, D), dtype=torch.uint8, device=x.device)
 
@@ -245,7 +250,7 @@ def scan_fwd(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Ten
         assert gate_bias.shape == (2, D) and gate_bias.dtype == torch.float32, "gate_bias: [2, D] fp32"
         gate_bias = gate_bias.contiguous()
     h = torch.empty_like(x)
-    nsub = lib.hawk_scan_split_chunks(B, T, D, 0)
+    nsub = _split_chunks(lib, x, 0)
     if nsub > 1:  # few (sequence, channel group) pairs: cut the sequences so that every SM gets work
         ws = _split_workspace(lib, x, B, nsub, D)
         with _on(x, "scan_fwd_split", 3):
@@ -284,7 +289,7 @@ def scan_bwd(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torch.Ten
         h0 = h0.contiguous()
     if gate_bias is not None:
         gate_bias = gate_bias.contiguous()
-    nsub = lib.hawk_scan_split_chunks(B, T, D, 2)
+    nsub = _split_chunks(lib, x, 2)
     if nsub > 1:
         ws = _split_workspace(lib, x, B, nsub, D)
         with _on(x, "scan_bwd_split", 5):
@@ -388,7 +393,7 @@ def scan_gelu_fwd(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam: torc
         assert gate_bias.shape == (2, D) and gate_bias.dtype == torch.float32, "gate_bias: [2, D] fp32"
         gate_bias = gate_bias.contiguous()
     h, out = torch.empty_like(x), torch.empty_like(x)
-    nsub = lib.hawk_scan_split_chunks(B, T, D, 1) if _split_view_ok(yv, T) else 1
+    nsub = _split_chunks(lib, x, 1) if _split_view_ok(yv, T) else 1
     if nsub > 1:
         ws = _split_workspace(lib, x, B, nsub, D)
         with _on(x, "scan_gelu_fwd_split", 3):
@@ -431,7 +436,7 @@ def scan_gelu_bwd_into(x: torch.Tensor, gx: torch.Tensor, ga: torch.Tensor, lam:
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
     if gate_bias is not None:
         gate_bias = gate_bias.contiguous()
-    nsub = lib.hawk_scan_split_chunks(B, T, D, 2) if (_split_view_ok(yv, T) and _split_view_ok(dy_out, T)) else 1
+    nsub = _split_chunks(lib, x, 3) if (_split_view_ok(yv, T) and _split_view_ok(dy_out, T)) else 1
     if nsub > 1:
         ws = _split_workspace(lib, x, B, nsub, D)
         with _on(x, "scan_gelu_bwd_split", 5):

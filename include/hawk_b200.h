@@ -116,7 +116,9 @@ int hawk_scan_gelu_bwd(const void* x, const void* gx, const void* ga, const floa
  * hawk_scan_split_workspace_bytes(B, nsub, D) bytes, no initialisation needed. */
 #define HAWK_SCAN_PASS_FWD 0      /* plain forward */
 #define HAWK_SCAN_PASS_FWD_GELU 1 /* forward with the gelu(y) * h epilogue */
-#define HAWK_SCAN_PASS_BWD 2      /* either backward */
+#define HAWK_SCAN_PASS_BWD 2      /* plain backward */
+#define HAWK_SCAN_PASS_BWD_GELU 3 /* backward with the epilogue */
+#define HAWK_SCAN_PASS_F32 8      /* added to one of these: fp32 storage (else bf16) */
 int hawk_scan_split_chunks(int B, int T, int D, int pass);
 size_t hawk_scan_split_workspace_bytes(int B, int nsub, int D);
 int hawk_scan_fwd_split(const void* x, const void* gx, const void* ga, const float* lam, const float* h0,

@@ -190,6 +190,24 @@ def test_time_split_policy_and_validation_need_no_gpu():
     assert lib.hawk_scan_fwd_split(p, p, p, p, None, None, p, 0, 0, p, None, 4, p, big, 1, 1024, 64, 1, None) < 0  # y without out
 
 
+def test_time_split_follows_length_and_type():
+    """Few channel groups are not enough: a short sequence stays whole (its launches would cost more than they save), a bf16
+    plain forward longest of all, fp32 with the epilogue shortest; the answers stay ones the entry points accept."""
+    lib = L.load()
+    F32 = 8
+    chunks = lambda T, D, which: lib.hawk_scan_split_chunks(1, T, D, which)  # noqa: E731
+    for which in range(4):
+        for dt in (0, F32):
+            assert chunks(512, 64, which + dt) == 1 and chunks(65536, 512, which + dt) > 1
+            for T in (512, 1024, 2048, 3072, 4096, 6144, 8192):
+                for D in (64, 512, 1024, 2048, 4096):
+                    n = chunks(T, D, which + dt)
+                    assert 1 <= n <= 64 and T % n == 0 and (n == 1 or T // n >= 256)
+    assert chunks(2048, 64, 0) == 1 and chunks(2048, 64, F32) > 1          # plain forward: bf16 18 / 19 us, fp32 41 / 28
+    assert chunks(1024, 64, 3) == 1 and chunks(1024, 64, 3 + F32) > 1      # fused backward: 30 / 30, 65 / 42
+    assert chunks(4096, 2048, 2) > 1 and chunks(4096, 2048, 2 + F32) == 1  # plain backward, 64 groups: 75 / 62, 103 / 116
+
+
 def test_reference_class_names_resolve_to_the_operators():
     """hawk/scan_fused.py:426-445 and hawk/fused_cross_entropy.py:11-79 expose their operators as
     `Class.apply`; the same spellings work here."""
