@@ -163,8 +163,10 @@ class _Operator(torch.library.CustomOpDef):
     def make(cls, name, mutates_args, fn):
         self = torch.library.custom_op(name, mutates_args=mutates_args)(fn)
         self.__class__ = cls
-        names = list(inspect.signature(fn).parameters)
+        parameters = inspect.signature(fn).parameters
+        names = list(parameters)
         self.direct, self.direct_fn, self.direct_autograd, self.direct_nargs = True, fn, None, len(names)
+        self.direct_defaults = tuple(p.default for p in parameters.values() if p.default is not p.empty)
         self.direct_mutated = [names.index(m) for m in mutates_args]
         self.__doc__, self.__name__ = fn.__doc__, fn.__name__
         return self
@@ -186,7 +188,10 @@ class _Operator(torch.library.CustomOpDef):
         self.direct_autograd = Function
 
     def __call__(self, *args, **kwargs):
-        if self.direct and not kwargs and len(args) == self.direct_nargs:
+        missing = self.direct_nargs - len(args)
+        if self.direct and not kwargs and 0 <= missing <= len(self.direct_defaults):
+            if missing:
+                args += self.direct_defaults[-missing:]
             record = _plain_call(args)
             if record is False:
                 out = self.direct_fn(*args)

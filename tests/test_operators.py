@@ -82,6 +82,21 @@ def test_a_registered_kernel_is_used(monkeypatch):
     assert torch.equal(twice(x), 3 * x)
 
 
+def test_defaults_left_out(monkeypatch):
+    @ops._operator("hawk_b200_test::affine", mutates_args=())
+    def affine(x: torch.Tensor, a: float = 2.0, b: float = 1.0) -> torch.Tensor:
+        return a * x + b
+    x = torch.ones(3)
+    seen = []
+    for direct in (None, False):  # the dispatcher, the direct way
+        monkeypatch.setattr(ops, "_plain_call", lambda args: (seen.append(args[1:]), direct)[1])
+        assert [float(affine(x, *rest)[0]) for rest in ((), (3.0,), (3.0, 5.0))] == [3.0, 4.0, 8.0]
+        assert float(affine(x, b=5.0)[0]) == 7.0
+        with pytest.raises((TypeError, RuntimeError)):
+            affine()
+    assert seen == 2 * [(2.0, 1.0), (3.0, 1.0), (3.0, 5.0)]
+
+
 def test_a_registered_vmap_rule_is_used():
     @ops._operator("hawk_b200_test::thrice", mutates_args=())
     def thrice(x: torch.Tensor) -> torch.Tensor:
